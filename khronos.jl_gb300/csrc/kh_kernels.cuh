@@ -84,6 +84,7 @@ __device__ __forceinline__ bool dbg_in(long long idx, long long n, int site) {
   }
 void dbg_read_tma(unsigned long long* count, long long* index, int* site);
 void dbg_read_kernels(unsigned long long* count, long long* index, int* site);
+void dbg_read_lean(unsigned long long* count, long long* index, int* site);
 #else
 #define KH_IN(idx, n, site) true
 #endif
@@ -213,6 +214,22 @@ constexpr int kTmaY = KH_TMA_ROWS;
 constexpr int kTmaStages = KH_TMA_STAGES;
 constexpr int kTmaMinBlocks = KH_TMA_MIN_BLOCKS;
 
+// Reduced-state half-step (kh_lean.cu): tile of kLeanX × kLeanY cells, 8 bytes of
+// FP32 (16 of FP64) cells per thread, ring stages, resident CTAs per SM it is
+// compiled for, and how many planes ahead a lane in the x-CPML fetches its
+// auxiliaries into L2.  Measured on whole runs (ms: waveguide 320×192×128, 96
+// steps / closed box 216×200×168, 100 steps / 64³, 256 steps; this choice 15.99 /
+// 9.72 / 3.55): 4 FP32 cells per thread 16.83 / 9.81 / 3.98; five CTAs per SM
+// 16.22 / 10.21 / 3.55; two stages 15.99 / 10.08 / 3.57; 128 × 4 tiles 17.18 / 9.87 /
+// 5.09; 128 × 2 16.85 / 9.65 / 4.97; 64 × 2 16.31 / 9.78 / 3.75.
+constexpr int kLeanX = 64;
+constexpr int kLeanY = 4;
+constexpr int kLeanVN = 2;
+constexpr int kLeanStages = 3;
+constexpr int kLeanXpf = 3;
+template <typename T>
+constexpr int kLeanMinBlocks = sizeof(T) == 4 ? 6 : 3;
+
 // Tensor maps of one half-step over the padded layout (x = pitch, y = ny+2,
 // z = nz+2): the curl-source arrays with a box of (kTmaX + 16 bytes) ×
 // (kTmaY + 1) × 1 (x and y halo on the side the curl reads), the updated
@@ -262,9 +279,17 @@ void launch_half_step_tma(bool h_half, const HalfStepParams<T>& p, const TmaMaps
 template <typename T>
 int prepare_tma_kernels();
 
-// CTAs of the TMA-staged kernel resident on one SM (after prepare_tma_kernels).
+// Reduced-state half-step (kh_lean.cu) for the CUDA-path CPML stages; its maps
+// have boxes of kLeanY rows.  expand: the complete T, U, W from its state.
 template <typename T>
-int tma_resident_ctas();
+void launch_half_step_lean(bool h_half, const HalfStepParams<T>& p, const TmaMaps& maps, void* stream);
+template <typename T>
+void launch_expand_state(bool h_half, const HalfStepParams<T>& p, void* stream);
+template <typename T>
+int prepare_lean_kernels();
+// CTAs of the reduced-state kernel resident on one SM (after prepare).
+template <typename T>
+int lean_resident_ctas();
 
 // History recording: copy one component over a cell box (x fastest) into a
 // contiguous slot of a history buffer.

@@ -1,0 +1,417 @@
+// Reduced-state half-step kernel for sm_103a: plain cells, CPML cells with
+// the CUDA-path stages on the auxiliaries that do not follow from others
+// (kh_lean.cuh), and special cells left to the sparse passes.
+//
+// A CTA owns a tile of 64 × kLeanY cells and marches its z chunk, H downwards
+// and E upwards, so that the z neighbour of the curl is the plane the thread
+// has just computed and stays in registers: a plane needs one ring stage.  One
+// elected thread keeps kLeanStages planes of TMA tiles in flight (curl sources
+// with their x/y halo, updated components, m⁻¹).
+//
+// What bounds it: plain tiles run at the memory's rate (216×200×168 FP32 without
+// CPML: 48 µs a half-step for 262 MB, 5.5 TB/s); tiles in the CPML by the latency
+// of a plane (their auxiliaries' loads, then update, store and barrier) and its
+// instructions.  Against the complete cascade (T, U, W stored for every CPML cell)
+// a 320×192×128 step moves 771 instead of 970 MB, in 41 + 49 M instead of 64 + 66 M
+// warp instructions.
+//
+// Every mbarrier wait is bounded: after kSleepWaitLimit tries the thread records
+// KH_ERR_TIMEOUT, leaves its cells alone from then on, and the issuing thread
+// waits (bounded) for the copies it issued before the CTA ends.
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include "../../include/khronos_gb300.h"
+#include "kh_async.cuh"
+#include "kh_lean.cuh"
+
+namespace kh {
+
+#ifdef KH_DEBUG_BOUNDS
+KH_DBG_READER(dbg_read_lean)
+#endif
+
+namespace {
+
+template <typename T, bool PV>
+struct LeanGeom {
+  static constexpr int HX = 16 / int(sizeof(T));  // x halo of the curl-source box (16 bytes)
+  static constexpr int XO = xoff<T>();
+  static constexpr int AX = kLeanX + HX;
+  static constexpr int A_BYTES = AX * (kLeanY + 1) * int(sizeof(T));
+  static constexpr int A_ELEMS = ((A_BYTES + 127) / 128 * 128) / int(sizeof(T));
+  static constexpr int O_ELEMS = kLeanX * kLeanY;
+  static constexpr int STAGE = 3 * A_ELEMS + (PV ? 6 : 3) * O_ELEMS;  // A0..2, O0..2(, m0..2)
+  static constexpr size_t SMEM =
+      size_t(kLeanStages) * STAGE * sizeof(T) + kLeanX * sizeof(AxisCoef<T>) + kLeanStages * sizeof(uint64_t);
+};
+
+}  // namespace
+
+constexpr int kLeanThreads = kLeanY * kLeanX / kLeanVN;
+
+template <typename T, bool H, bool PV, bool STALL = false>
+__global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
+    half_step_lean_kernel(const __grid_constant__ HalfStepParams<T> p, const __grid_constant__ TmaMaps maps) {
+  using G = LeanGeom<T, PV>;
+  constexpr int VN = kLeanVN;
+  constexpr int LPR = kLeanX / VN;  // lanes per tile row
+  using PK = Pack<T, VN>;
+  constexpr int s = H ? 1 : -1;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  T* stages = reinterpret_cast<T*>(smem_raw);
+  AxisCoef<T>* xtab = reinterpret_cast<AxisCoef<T>*>(stages + kLeanStages * G::STAGE);  // per tile column: a, b, om, op
+  uint64_t* bars = reinterpret_cast<uint64_t*>(xtab + kLeanX);
+
+  const int tid = threadIdx.x;
+  const int col = (tid % LPR) * VN;
+  const int wy = tid / LPR;
+  const bool issuer = tid == 0;
+  const int x_tile = blockIdx.x * kLeanX;
+  const int y_tile = blockIdx.y * kLeanY;
+  const int j = y_tile + wy;
+  const int x0 = x_tile + col;
+  const bool lane_ok = j < p.ny && x0 < p.nx;
+  const bool full = x0 + VN <= p.nx;  // all VN cells exist
+  const int k0 = blockIdx.z * p.zplanes;
+  const int k1 = min(k0 + p.zplanes, p.nz);
+  const int N = k1 - k0;
+  constexpr int kLimit = STALL ? kStallSleepWaitLimit : kSleepWaitLimit;
+  const bool tfx = x_tile < p.pml_lo[0] || (p.pml_hi[0] > 0 && x_tile + kLeanX > p.nx - p.pml_hi[0]);
+  const bool tfy = y_tile < p.pml_lo[1] || (p.pml_hi[1] > 0 && y_tile + kLeanY > p.ny - p.pml_hi[1]);
+
+  if (issuer) {
+    for (int st = 0; st < kLeanStages; ++st) mbar_init(&bars[st], 1);
+    mbar_fence_init();
+  }
+  if (tfx)
+    for (int c = tid; c < kLeanX; c += kLeanThreads) {
+      const int i = x_tile + c;
+      const bool f = i < p.nx && (i < p.pml_lo[0] || i >= p.nx - p.pml_hi[0]);
+      const RedAxis<T> r = red_axis<T>(f && KH_IN(i, p.nx, 2120) ? p.ax[0][i] : AxisCoef<T>{}, f);
+      xtab[c] = {r.a, r.b, r.om, r.op};
+    }
+  __syncthreads();
+
+  // load n: the tiles of the n-th plane of the march
+  auto issue = [&](int n, int st) {
+    T* dst = stages + st * G::STAGE;
+    const int k = H ? k1 - 1 - n : k0 + n;
+    if (STALL && n == 0) {
+      // failure-detection test instantiation: the first stage expects 16 bytes
+      // and no copy is issued into it, so the wait on it runs out and nothing
+      // is left in flight when the CTA returns
+      mbar_arrive_expect_tx(&bars[st], 16u);
+      return;
+    }
+    mbar_arrive_expect_tx(&bars[st], 3u * uint32_t(G::A_BYTES) + (PV ? 6u : 3u) * uint32_t(G::O_ELEMS * sizeof(T)));
+    const int zc = k + 1;                                        // padded plane index
+    const int ax = H ? G::XO + x_tile : G::XO - G::HX + x_tile;  // padded x of the A box
+    const int ay = H ? 1 + y_tile : y_tile;                      // padded y of the A box
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      tma_load_3d(dst + c * G::A_ELEMS, &maps.a[c], ax, ay, zc, &bars[st]);
+      tma_load_3d(dst + 3 * G::A_ELEMS + c * G::O_ELEMS, &maps.o[c], G::XO + x_tile, 1 + y_tile, zc, &bars[st]);
+      if constexpr (PV)
+        tma_load_3d(dst + 3 * G::A_ELEMS + (3 + c) * G::O_ELEMS, &maps.m[c], G::XO + x_tile, 1 + y_tile, zc,
+                    &bars[st]);
+    }
+    // the plane's y/z auxiliaries into L2 ahead of the register loads (the
+    // x ones, a few columns of the tile, are fetched by their own lanes)
+    const bool tfz = k < p.pml_lo[2] || k >= p.nz - p.pml_hi[2];
+    if (tfy) tma_prefetch_3d(&maps.t[1], G::XO + x_tile, 1 + y_tile, zc);
+    if (tfz) tma_prefetch_3d(&maps.t[2], G::XO + x_tile, 1 + y_tile, zc);
+    if (tfy && tfz) tma_prefetch_3d(&maps.u[0], G::XO + x_tile, 1 + y_tile, zc);
+  };
+  if (issuer) {
+    const int first = min(kLeanStages, N);
+    for (int n = 0; n < first; ++n) issue(n, n);
+  }
+
+  const long long step = H ? -p.plane : p.plane;
+  long long q = p.origin + (long long)(H ? k1 - 1 : k0) * p.plane + (long long)j * p.pitch + x0;
+  T *o0 = p.O[0] + q, *o1 = p.O[1] + q, *o2 = p.O[2] + q;
+  auto get = [&](const T* arr, int site) -> PK {
+    return KH_IN(q, p.total, site) && KH_IN(q + VN - 1, p.total, site) ? *reinterpret_cast<const PK*>(arr + q) : PK{};
+  };
+  auto put = [&](T* a, const PK& x, int site) {
+    if (full) {
+      if (KH_IN(q, p.total, site) && KH_IN(q + VN - 1, p.total, site)) *reinterpret_cast<PK*>(a) = x;
+    } else {
+#pragma unroll
+      for (int v = 0; v < VN - 1; ++v)
+        if (x0 + v < p.nx && KH_IN(q + v, p.total, site)) a[v] = x.v[v];
+    }
+  };
+  // the z neighbour plane of the first plane of the march
+  PK nb0{}, nb1{};
+  if (lane_ok) {
+    const long long qn = q - step;
+    if (KH_IN(qn, p.total, 2101) && KH_IN(qn + VN - 1, p.total, 2102)) {
+      nb0 = *reinterpret_cast<const PK*>(p.A[0] + qn);
+      nb1 = *reinterpret_cast<const PK*>(p.A[1] + qn);
+    }
+  }
+  const bool fy = lane_ok && (j < p.pml_lo[1] || j >= p.ny - p.pml_hi[1]);
+  const RedAxis<T> ry = red_axis<T>(fy && KH_IN(j, p.ny, 2111) ? p.ax[1][j] : AxisCoef<T>{}, fy);
+  bool fxv[VN], anyfx = false;
+#pragma unroll
+  for (int v = 0; v < VN; ++v) {
+    const int i = x0 + v;
+    fxv[v] = tfx && lane_ok && i < p.nx && (i < p.pml_lo[0] || i >= p.nx - p.pml_hi[0]);
+    anyfx |= fxv[v];
+  }
+  // special-cell plane bits of this row segment, one word per 64 planes
+  const long long tb_group = (long long)p.ny * p.nxb;
+  const long long tb_row = (long long)j * p.nxb + (x0 >> 6);
+  auto tile_word = [&](int g) -> uint64_t {
+    return (p.tile_bits && lane_ok && KH_IN(tb_row + g * tb_group, p.n_tile_words, 2103))
+               ? p.tile_bits[tb_row + g * tb_group] : 0ull;
+  };
+  // the bit of the current plane is the top (H) or the bottom (E) one
+  int k = H ? k1 - 1 : k0;
+  auto tile_bits_from = [&](int kk) -> uint64_t {
+    const uint64_t w = tile_word(kk >> 6);
+    return H ? w << (63 - (kk & 63)) : w >> (kk & 63);
+  };
+  uint64_t tbits = tile_bits_from(k);
+  const int a = (H ? wy : wy + 1) * G::AX + (H ? 0 : G::HX) + col;
+  const int ob = wy * kLeanX + col;
+  const T cd0 = p.cd[0], cd1 = p.cd[1], cd2 = p.cd[2];
+  int gave_up = -1;  // the plane at which this thread's wait ran out
+  int st = 0;        // ring stage of load n, and the parity of its phase
+  uint32_t parity = 0;
+  for (int n = 0; n < N; ++n) {
+    const bool fz = k < p.pml_lo[2] || k >= p.nz - p.pml_hi[2];
+    const bool tf = H ? (tbits >> 63) != 0 : (tbits & 1ull) != 0;
+    const bool plain = !(anyfx || fy || fz || tf);
+    // auxiliaries: T in the own-axis CPML, U in those of both other axes; rows
+    // with special cells take all of them
+    Cells<T, VN> t, u;
+    AxisCoef<T> cz{};
+    if (!plain && lane_ok) {
+      if (anyfx || tf) t.c[0] = get(p.Ts[0], 2104);
+      if (fy || tf) t.c[1] = get(p.Ts[1], 2105);
+      if (fz || tf) t.c[2] = get(p.Ts[2], 2106);
+      if (fy && (fz || tf)) u.c[0] = get(p.U[0], 2107);
+      if (fz && (anyfx || tf)) u.c[1] = get(p.U[1], 2108);
+      if (anyfx && (fy || tf)) u.c[2] = get(p.U[2], 2109);
+      if (fz && KH_IN(k, p.nz, 2112)) cz = p.ax[2][k];
+      if (anyfx && n + kLeanXpf < N) {
+        const long long qp = q + kLeanXpf * step;
+        if (KH_IN(qp + VN - 1, p.total, 2113)) {
+          l2_prefetch(p.Ts[0] + qp);
+          if (fz) l2_prefetch(p.U[1] + qp);
+          if (fy) l2_prefetch(p.U[2] + qp);
+        }
+      }
+    }
+    if (gave_up < 0 && !mbar_wait_sleep(smem_u32(bars + st), parity, kLimit)) {
+      gave_up = n;
+      if (p.err) atomicExch(p.err, KH_ERR_TIMEOUT);
+    }
+    const bool smem_ok = KH_IN(a + (H ? 0 : -1), G::A_ELEMS, 2114) && KH_IN(a + (H ? VN : VN - 1), G::A_ELEMS, 2115) &&
+                         KH_IN(a + s * G::AX, G::A_ELEMS, 2116) && KH_IN(a + s * G::AX + VN - 1, G::A_ELEMS, 2117) &&
+                         KH_IN(ob + VN - 1, G::O_ELEMS, 2118);
+    if (gave_up < 0 && lane_ok && smem_ok) {
+      const T* A0 = stages + st * G::STAGE + a;
+      const T* A1 = A0 + G::A_ELEMS;
+      const T* A2 = A1 + G::A_ELEMS;
+      const T* Os = stages + st * G::STAGE + 3 * G::A_ELEMS + ob;
+      auto lds = [](const T* q) { return *reinterpret_cast<const PK*>(q); };
+      const PK c0 = lds(A0), c1 = lds(A1), c2 = lds(A2), y0 = lds(A0 + s * G::AX), y2 = lds(A2 + s * G::AX);
+      const T e1 = A1[H ? VN : -1], e2 = A2[H ? VN : -1];  // x neighbours past the thread's cells
+      Cells<T, VN> O, m, K;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        O.c[c] = lds(Os + c * G::O_ELEMS);
+        if constexpr (PV) {
+          m.c[c] = lds(Os + (3 + c) * G::O_ELEMS);
+        } else {
+#pragma unroll
+          for (int v = 0; v < VN; ++v) m.c[c].v[v] = p.m_scalar;
+        }
+      }
+#pragma unroll
+      for (int v = 0; v < VN; ++v) {
+        // forward difference (H): cell v reads x + 1; backward (E): x - 1
+        const T x1 = H ? (v + 1 < VN ? c1.v[(v + 1) % VN] : e1) : (v > 0 ? c1.v[(v + VN - 1) % VN] : e1);
+        const T x2 = H ? (v + 1 < VN ? c2.v[(v + 1) % VN] : e2) : (v > 0 ? c2.v[(v + VN - 1) % VN] : e2);
+        K.c[0].v[v] = curl_rn(cd2, nb1.v[v], c1.v[v], cd1, y2.v[v], c2.v[v]);
+        K.c[1].v[v] = curl_rn(cd0, x2, c2.v[v], cd2, nb0.v[v], c0.v[v]);
+        K.c[2].v[v] = curl_rn(cd1, y0.v[v], c0.v[v], cd0, x1, c1.v[v]);
+      }
+      nb0 = c0;
+      nb1 = c1;
+      if (plain) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+          for (int v = 0; v < VN; ++v) O.c[c].v[v] = fma_rn(m.c[c].v[v], K.c[c].v[v], O.c[c].v[v]);
+      } else {
+        const RedAxis<T> rz = red_axis<T>(cz, fz);
+        bool sp[VN], anysp = false;
+        if (tf) {
+          constexpr uint32_t kSp = H ? kSpecialH : kSpecialE;
+#pragma unroll
+          for (int v = 0; v < VN; ++v) {
+            sp[v] = x0 + v < p.nx && KH_IN(q + v, p.total, 2110) && (p.cell_class[q + v] & kSp) != 0;
+            anysp |= sp[v];
+          }
+        }
+        if (!anysp) {
+          update_cells<T, VN>(fxv, anyfx, xtab + col, ry, rz, K, m, O, t, u);
+        } else {
+          Cells<T, VN> w;
+          if (anyfx) w.c[0] = get(p.W[0], 2128);
+          if (fy) w.c[1] = get(p.W[1], 2129);
+          if (fz) w.c[2] = get(p.W[2], 2119);
+          update_special_cells<T, VN>(sp, fxv, p.ax[0] + x0, p.ax[1] + j, cz.s, xtab + col, ry, rz, K, m, O, t, u, w);
+          if (anyfx) put(p.W[0] + q, w.c[0], 2131);
+          if (fy) put(p.W[1] + q, w.c[1], 2132);
+          if (fz) put(p.W[2] + q, w.c[2], 2133);
+        }
+        // what was loaded goes back (values that a cell does not use unchanged)
+        if (anyfx || tf) put(p.Ts[0] + q, t.c[0], 2121);
+        if (fy || tf) put(p.Ts[1] + q, t.c[1], 2122);
+        if (fz || tf) put(p.Ts[2] + q, t.c[2], 2123);
+        if (fy && (fz || tf)) put(p.U[0] + q, u.c[0], 2124);
+        if (fz && (anyfx || tf)) put(p.U[1] + q, u.c[1], 2125);
+        if (anyfx && (fy || tf)) put(p.U[2] + q, u.c[2], 2126);
+      }
+      if (full) {
+        if (KH_IN(q, p.total, 2127) && KH_IN(q + VN - 1, p.total, 2127)) {
+          *reinterpret_cast<PK*>(o0) = O.c[0];
+          *reinterpret_cast<PK*>(o1) = O.c[1];
+          *reinterpret_cast<PK*>(o2) = O.c[2];
+        }
+      } else {
+        put(o0, O.c[0], 2127);
+        put(o1, O.c[1], 2127);
+        put(o2, O.c[2], 2127);
+      }
+    }
+    q += step;
+    o0 += step;
+    o1 += step;
+    o2 += step;
+    // every thread is done with load n: its stage takes load n + kLeanStages
+    __syncthreads();
+    if (issuer && gave_up < 0 && n + kLeanStages < N) {
+      fence_proxy_async();
+      issue(n + kLeanStages, st);
+    }
+    if (++st == kLeanStages) {
+      st = 0;
+      parity ^= 1u;
+    }
+    k += H ? -1 : 1;
+    tbits = H ? tbits << 1 : tbits >> 1;
+    if ((k & 63) == (H ? 63 : 0) && n + 1 < N) tbits = tile_bits_from(k);
+  }
+  // an issuer that gave up waits (bounded) for the copies it has in flight
+  if (issuer && gave_up >= 0)
+    for (int l = gave_up; l < min(gave_up + kLeanStages, N); ++l)
+      mbar_wait_sleep(smem_u32(bars + l % kLeanStages), uint32_t((l / kLeanStages) & 1), kLimit);
+}
+
+// ---------------------------------------------------------------------------
+// The complete T, U, W of every CPML cell from the reduced state, for state
+// files and for the general kernel (kh_lean.cuh says how they follow).
+template <typename T, bool H>
+__global__ void expand_state_kernel(const HalfStepParams<T> p) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
+  if (i >= p.nx) return;
+  const bool f[3] = {i < p.pml_lo[0] || i >= p.nx - p.pml_hi[0], j < p.pml_lo[1] || j >= p.ny - p.pml_hi[1],
+                     k < p.pml_lo[2] || k >= p.nz - p.pml_hi[2]};
+  if (!(f[0] || f[1] || f[2])) return;
+  const long long q = p.origin + (long long)k * p.plane + (long long)j * p.pitch + i;
+  if (!KH_IN(q, p.total, 2130)) return;
+  if (p.cell_class && (p.cell_class[q] & (H ? kSpecialH : kSpecialE))) return;  // keeps the complete state
+  const int idx[3] = {i, j, k};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const int n = (c + 1) % 3, v = (c + 2) % 3;
+    const T m = p.m_inv[c] ? p.m_inv[c][q] : p.m_scalar;
+    const T t = f[c] ? p.Ts[c][q] : (m != T(0) ? p.O[c][q] / m : T(0));
+    p.Ts[c][q] = t;
+    if (f[n] && !f[v]) p.U[c][q] = p.ax[n][idx[n]].s != T(0) ? t : T(0);
+    if (f[c]) p.W[c][q] = p.ax[c][idx[c]].s != T(0) ? mul_rn(m, t) : T(0);
+  }
+}
+
+template <typename T>
+void launch_expand_state(bool h_half, const HalfStepParams<T>& p, void* stream) {
+  const dim3 grid((p.nx + 127) / 128, p.ny, p.nz);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (h_half) expand_state_kernel<T, true><<<grid, 128, 0, st>>>(p);
+  else expand_state_kernel<T, false><<<grid, 128, 0, st>>>(p);
+}
+
+template <typename T, bool H, bool PV>
+static void launch_lean_variant(const HalfStepParams<T>& p, const TmaMaps& maps, cudaStream_t st) {
+  const dim3 block(kLeanThreads, 1, 1);
+  const dim3 grid((p.nx + kLeanX - 1) / kLeanX, (p.ny + kLeanY - 1) / kLeanY, (p.nz + p.zplanes - 1) / p.zplanes);
+  if constexpr (sizeof(T) == 4) {
+    if (p.stall_tx) {  // failure-detection test instantiation (FP32 only)
+      half_step_lean_kernel<T, H, PV, true><<<grid, block, LeanGeom<T, PV>::SMEM, st>>>(p, maps);
+      return;
+    }
+  }
+  half_step_lean_kernel<T, H, PV><<<grid, block, LeanGeom<T, PV>::SMEM, st>>>(p, maps);
+}
+
+template <typename T>
+void launch_half_step_lean(bool h_half, const HalfStepParams<T>& p, const TmaMaps& maps, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const bool pv = p.m_inv[0] != nullptr;
+  if (h_half) {
+    if (pv) launch_lean_variant<T, true, true>(p, maps, st);
+    else launch_lean_variant<T, true, false>(p, maps, st);
+  } else {
+    if (pv) launch_lean_variant<T, false, true>(p, maps, st);
+    else launch_lean_variant<T, false, false>(p, maps, st);
+  }
+}
+
+template <typename T, bool H, bool PV, bool STALL = false>
+static int set_lean_attr() {
+  return int(cudaFuncSetAttribute(half_step_lean_kernel<T, H, PV, STALL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(LeanGeom<T, PV>::SMEM)));
+}
+
+template <typename T>
+int prepare_lean_kernels() {
+  int e = 0;
+  e |= set_lean_attr<T, true, true>();
+  e |= set_lean_attr<T, true, false>();
+  e |= set_lean_attr<T, false, true>();
+  e |= set_lean_attr<T, false, false>();
+  if constexpr (sizeof(T) == 4) {
+    e |= set_lean_attr<T, true, true, true>();
+    e |= set_lean_attr<T, true, false, true>();
+    e |= set_lean_attr<T, false, true, true>();
+    e |= set_lean_attr<T, false, false, true>();
+  }
+  return e;
+}
+
+template <typename T>
+int lean_resident_ctas() {
+  int n = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, half_step_lean_kernel<T, false, true>, kLeanThreads,
+                                                    LeanGeom<T, true>::SMEM) != cudaSuccess)
+    return 1;
+  return n > 0 ? n : 1;
+}
+
+template void launch_half_step_lean<float>(bool, const HalfStepParams<float>&, const TmaMaps&, void*);
+template void launch_half_step_lean<double>(bool, const HalfStepParams<double>&, const TmaMaps&, void*);
+template void launch_expand_state<float>(bool, const HalfStepParams<float>&, void*);
+template void launch_expand_state<double>(bool, const HalfStepParams<double>&, void*);
+template int prepare_lean_kernels<float>();
+template int prepare_lean_kernels<double>();
+template int lean_resident_ctas<float>();
+template int lean_resident_ctas<double>();
+
+}  // namespace kh

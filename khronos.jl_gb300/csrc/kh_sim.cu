@@ -834,6 +834,11 @@ class Sim : public SimBase {
       // else the FULL launch while sources are active
       if (src_on_dispersive_ && !disp_fix_) src_lean_ok_[0] = false;
     }
+    if (use_tma_ && d_.semantics == KH_SEM_CPML) {
+      const bool dispersive = chi3_ != nullptr || !poles_d_.empty();
+      reduced_[0] = !(msigd_[0] || msigd_[1] || msigd_[2]) && (!dispersive || disp_fix_);
+      reduced_[1] = !(msigb_[0] || msigb_[1] || msigb_[2]);
+    }
     prepared_ = true;
     return KH_OK;
 #undef KH_TRY
@@ -1043,6 +1048,16 @@ class Sim : public SimBase {
     for (int a = 0; a < 3; ++a)
       if (dm[a] <= 0 || st[a] < 0 || st[a] + dm[a] > n_[a]) return fail(KH_ERR_INVALID, "box outside the grid");
     if (kh_status es = wait_idle(); es != KH_OK) return es;
+    // mid-run in a CPML cell of a half on the reduced state: W keeps the old
+    // material's value for one step, so the run goes on from the complete state
+    if (timestep_ > 0 && reduced_[kind == KH_MAT_MU_INV ? 1 : 0] && !complete_state_) {
+      bool cpml = false;
+      for (int a = 0; a < 3; ++a) cpml = cpml || st[a] < lo_[a] || st[a] + dm[a] > n_[a] - hi_[a];
+      if (cpml) {
+        if (kh_status es = expand_state(); es != KH_OK) return es;
+        complete_state_ = true;
+      }
+    }
     std::vector<T> plane(size_t(dm[0]) * dm[1]);
     for (int k = 0; k < dm[2]; ++k) {
       for (int j = 0; j < dm[1]; ++j)
@@ -1154,6 +1169,7 @@ class Sim : public SimBase {
     KH_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     timestep_ = 0;
     sources_active_ = true;
+    complete_state_ = false;
     return KH_OK;
   }
 
@@ -1166,8 +1182,10 @@ class Sim : public SimBase {
   kh_status export_state(void* dst, int64_t bytes) override {
     if (!prepared_ || !dst || bytes != state_bytes()) return fail(KH_ERR_INVALID, "bad export buffer");
     if (kh_status es = wait_idle(); es != KH_OK) return es;
+    if (kh_status es = expand_state(); es != KH_OK) return es;
     char* p = static_cast<char*>(dst);
-    int64_t hdr[2] = {timestep_, sources_active_ ? 1 : 0};
+    // bit 0: sources active, bit 1: the run goes on from the complete state
+    int64_t hdr[2] = {timestep_, (sources_active_ ? 1 : 0) | (complete_state_ ? 2 : 0)};
     std::memcpy(p, hdr, 16);
     p += 16;
     for (auto& s : state_) {
@@ -1189,7 +1207,8 @@ class Sim : public SimBase {
       p += s.second;
     }
     timestep_ = hdr[0];
-    sources_active_ = hdr[1] != 0;
+    sources_active_ = (hdr[1] & 1) != 0;
+    complete_state_ = (hdr[1] & 2) != 0 && (reduced_[0] || reduced_[1]);
     return KH_OK;
   }
 
@@ -1223,16 +1242,19 @@ class Sim : public SimBase {
       }
       if (cnt == 0 || !(f[0] || f[1] || f[2])) continue;
       // Σ_c 2·(U_c + W_c + T_c): T_c = U_c ∨ W_c on the CPU path; the CUDA-path
-      // stages also keep T_c where only the prev axis is PML (σ_prev stage).
+      // stages also keep T_c where only the prev axis is PML (σ_prev stage).  The
+      // reduced state keeps T_c on the own axis and U_c where both others meet.
       const bool cpml = d_.semantics == KH_SEM_CPML;
-      int aux = 0;
-      for (int c = 0; c < 3; ++c) {
-        const int u = f[(c + 1) % 3] ? 1 : 0, w = f[c] ? 1 : 0;
-        const int t = (u || w || (cpml && f[(c + 2) % 3])) ? 1 : 0;
-        aux += 2 * (u + w + t);
+      for (int h = 0; h < 2; ++h) {
+        int aux = 0;
+        for (int c = 0; c < 3; ++c) {
+          const bool n = f[(c + 1) % 3], v = f[(c + 2) % 3];
+          const int u = (reduced_[h] ? n && v : n) ? 1 : 0, w = !reduced_[h] && f[c] ? 1 : 0;
+          const int t = (reduced_[h] ? f[c] : u || w || (cpml && v)) ? 1 : 0;
+          aux += 2 * (u + w + t);
+        }
+        (h ? hw : ew) += double(aux) * double(cnt);
       }
-      hw += double(aux) * double(cnt);  // B side
-      ew += double(aux) * double(cnt);  // D side
     }
     if (!chi3_h_.empty() || !poles_.empty()) {
       const size_t ncenter = size_t(n_[0]) * n_[1] * n_[2];
@@ -1575,11 +1597,11 @@ class Sim : public SimBase {
     const bool msb = msigb_[0] || msigb_[1] || msigb_[2];
     const bool msd = msigd_[0] || msigd_[1] || msigd_[2];
     const bool ref_cpu = d_.semantics == KH_SEM_REFERENCE_CPU;
-    const bool full_h_base = msb || (ref_cpu && special_in_region_[1]);
+    const bool full_h_base = msb || (ref_cpu && special_in_region_[1]) || complete_state_;
     // χ3 and pole cells: in the LEAN E launch plus the dispersive-cell pass
     // (disp_fix_), or in the FULL launch
     const bool dispersive = chi3_ != nullptr || !poles_d_.empty();
-    const bool full_e_base = msd || (dispersive && !disp_fix_) || (ref_cpu && special_in_region_[0]);
+    const bool full_e_base = msd || (dispersive && !disp_fix_) || (ref_cpu && special_in_region_[0]) || complete_state_;
     const kh::WrapParams<T> wh = wrap_params(true), we = wrap_params(false);
     kh::SourceFixParams<T> fh = fix_params(true), fe = fix_params(false);
     kh::DispFixParams<T> dfix = disp_params(pe);
@@ -1591,7 +1613,8 @@ class Sim : public SimBase {
       const bool src_h = P.sa && has_src_[1];
       ph.full = (full_h_base || (src_h && !src_lean_ok_[1])) ? 1 : 0;
       mark(s, 0);
-      if (use_tma_) kh::launch_half_step_tma<T>(true, ph, maps_h_, st);
+      if (reduced_[1] && !ph.full) kh::launch_half_step_lean<T>(true, ph, lean_maps_h_, st);
+      else if (use_tma_) kh::launch_half_step_tma<T>(true, ph, maps_h_, st);
       else kh::launch_half_step<T>(true, ph, st);
       ++launches;
       if (src_h && !ph.full) {
@@ -1611,7 +1634,8 @@ class Sim : public SimBase {
       pe.f_now = dtab + P.fE;
       const bool src_e = P.sa && has_src_[0];
       pe.full = (full_e_base || (src_e && !src_lean_ok_[0])) ? 1 : 0;
-      if (use_tma_) kh::launch_half_step_tma<T>(false, pe, maps_e_, st);
+      if (reduced_[0] && !pe.full) kh::launch_half_step_lean<T>(false, pe, lean_maps_e_, st);
+      else if (use_tma_) kh::launch_half_step_tma<T>(false, pe, maps_e_, st);
       else kh::launch_half_step<T>(false, pe, st);
       ++launches;
       if (src_e && !pe.full) {
@@ -1644,6 +1668,7 @@ class Sim : public SimBase {
       sig.reserve(size_t(nb) * 8 + 4);
       sig.push_back(nb);
       sig.push_back(b);
+      sig.push_back(complete_state_ ? 1 : 0);
       for (int q = 0; q < nb; ++q) {
         const StepPlan& P = plan[q];
         sig.push_back(P.sa ? 1 : 0);
@@ -1848,6 +1873,28 @@ class Sim : public SimBase {
     ++launches;
   }
 
+  // Tensor map of one padded full-domain array with the given box.
+  kh_status encode_map(CUtensorMap* m, T* base, const cuuint32_t* box) {
+    static std::atomic<void*> entry{nullptr};  // the driver's function, the same for every device
+    void* fn = entry.load();
+    if (!fn) {
+      cudaDriverEntryPointQueryResult qr;
+      KH_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &qr));
+      if (!fn || qr != cudaDriverEntryPointSuccess) return fail(KH_ERR_CUDA, "cuTensorMapEncodeTiled not available");
+      entry = fn;
+    }
+    auto encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+    const cuuint64_t dims[3] = {cuuint64_t(pitch_), cuuint64_t(n_[1] + 2), cuuint64_t(n_[2] + 2)};
+    const cuuint64_t strides[2] = {cuuint64_t(pitch_) * sizeof(T), cuuint64_t(plane_) * sizeof(T)};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUtensorMapDataType dt = sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
+    const CUresult r = encode(m, dt, 3, static_cast<void*>(base), dims, strides, box, estr,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(KH_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+    return KH_OK;
+  }
+
   // Tensor maps over the padded layout for the TMA-staged kernel.
   kh_status build_tma_maps() {
     // the attribute is per device: set it once for each device a simulation runs on
@@ -1856,49 +1903,40 @@ class Sim : public SimBase {
     KH_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= kMaxDevices) return fail(KH_ERR_UNSUPPORTED, "device ordinal above the supported range");
     if (!attr_done[dev]) {
-      if (kh::prepare_tma_kernels<T>() != 0)
+      if (kh::prepare_tma_kernels<T>() != 0 || kh::prepare_lean_kernels<T>() != 0)
         return fail(KH_ERR_CUDA, "cudaFuncSetAttribute on the TMA half-step kernels failed");
       attr_done[dev] = true;
     }
     int sms = 0;
     KH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    tma_slots_ = sms * kh::tma_resident_ctas<T>();
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult qr;
-    KH_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &qr));
-    if (!fn || qr != cudaDriverEntryPointSuccess) return fail(KH_ERR_CUDA, "cuTensorMapEncodeTiled not available");
-    auto encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+    tma_slots_ = sms * kh::lean_resident_ctas<T>();
     const int hx = 16 / int(sizeof(T));
-    const cuuint64_t dims[3] = {cuuint64_t(pitch_), cuuint64_t(n_[1] + 2), cuuint64_t(n_[2] + 2)};
-    const cuuint64_t strides[2] = {cuuint64_t(pitch_) * sizeof(T), cuuint64_t(plane_) * sizeof(T)};
-    const cuuint32_t box_a[3] = {cuuint32_t(kh::kTmaX + hx), cuuint32_t(kh::kTmaY + 1), 1};
-    const cuuint32_t box_o[3] = {cuuint32_t(kh::kTmaX), cuuint32_t(kh::kTmaY), 1};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUtensorMapDataType dt = sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
-    auto mk = [&](CUtensorMap* m, T* base, const cuuint32_t* box) -> kh_status {
-      // base points at element (-1,-1,-1) - XOFF + ... : the allocation start
-      CUresult r = encode(m, dt, 3, static_cast<void*>(base), dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      if (r != CUDA_SUCCESS) return fail(KH_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-      return KH_OK;
+    struct MapSet {
+      kh::TmaMaps *h, *e;
+      int cols, rows;
     };
-    std::memset(&maps_h_, 0, sizeof(maps_h_));
-    std::memset(&maps_e_, 0, sizeof(maps_e_));
-    for (int c = 0; c < 3; ++c) {
-      kh_status st;
-      if ((st = mk(&maps_h_.a[c], E_[c], box_a)) != KH_OK) return st;
-      if ((st = mk(&maps_h_.o[c], H_[c], box_o)) != KH_OK) return st;
-      if (mu_[c] && (st = mk(&maps_h_.m[c], mu_[c], box_o)) != KH_OK) return st;
-      if ((st = mk(&maps_e_.a[c], H_[c], box_a)) != KH_OK) return st;
-      if ((st = mk(&maps_e_.o[c], E_[c], box_o)) != KH_OK) return st;
-      if (eps_[c] && (st = mk(&maps_e_.m[c], eps_[c], box_o)) != KH_OK) return st;
-      if (B_[c] && (st = mk(&maps_h_.t[c], B_[c], box_o)) != KH_OK) return st;
-      if (UB_[c] && (st = mk(&maps_h_.u[c], UB_[c], box_o)) != KH_OK) return st;
-      if (WB_[c] && (st = mk(&maps_h_.w[c], WB_[c], box_o)) != KH_OK) return st;
-      if (D_[c] && (st = mk(&maps_e_.t[c], D_[c], box_o)) != KH_OK) return st;
-      if (UD_[c] && (st = mk(&maps_e_.u[c], UD_[c], box_o)) != KH_OK) return st;
-      if (WD_[c] && (st = mk(&maps_e_.w[c], WD_[c], box_o)) != KH_OK) return st;
+    for (const MapSet& ms : {MapSet{&maps_h_, &maps_e_, kh::kTmaX, kh::kTmaY},
+                             MapSet{&lean_maps_h_, &lean_maps_e_, kh::kLeanX, kh::kLeanY}}) {
+      const cuuint32_t box_a[3] = {cuuint32_t(ms.cols + hx), cuuint32_t(ms.rows + 1), 1};
+      const cuuint32_t box_o[3] = {cuuint32_t(ms.cols), cuuint32_t(ms.rows), 1};
+      kh::TmaMaps &maps_h = *ms.h, &maps_e = *ms.e;
+      std::memset(&maps_h, 0, sizeof(maps_h));
+      std::memset(&maps_e, 0, sizeof(maps_e));
+      for (int c = 0; c < 3; ++c) {
+        kh_status st;
+        if ((st = encode_map(&maps_h.a[c], E_[c], box_a)) != KH_OK) return st;
+        if ((st = encode_map(&maps_h.o[c], H_[c], box_o)) != KH_OK) return st;
+        if (mu_[c] && (st = encode_map(&maps_h.m[c], mu_[c], box_o)) != KH_OK) return st;
+        if ((st = encode_map(&maps_e.a[c], H_[c], box_a)) != KH_OK) return st;
+        if ((st = encode_map(&maps_e.o[c], E_[c], box_o)) != KH_OK) return st;
+        if (eps_[c] && (st = encode_map(&maps_e.m[c], eps_[c], box_o)) != KH_OK) return st;
+        if (B_[c] && (st = encode_map(&maps_h.t[c], B_[c], box_o)) != KH_OK) return st;
+        if (UB_[c] && (st = encode_map(&maps_h.u[c], UB_[c], box_o)) != KH_OK) return st;
+        if (WB_[c] && (st = encode_map(&maps_h.w[c], WB_[c], box_o)) != KH_OK) return st;
+        if (D_[c] && (st = encode_map(&maps_e.t[c], D_[c], box_o)) != KH_OK) return st;
+        if (UD_[c] && (st = encode_map(&maps_e.u[c], UD_[c], box_o)) != KH_OK) return st;
+        if (WD_[c] && (st = encode_map(&maps_e.w[c], WD_[c], box_o)) != KH_OK) return st;
+      }
     }
     return KH_OK;
   }
@@ -1914,11 +1952,25 @@ class Sim : public SimBase {
     // SMs); shallower when the launch would not fill two rounds of resident CTAs.
     int z = 10;
     if (use_tma_ && tma_slots_ > 0) {
-      const long long xy = (long long)((n_[0] + kh::kTmaX - 1) / kh::kTmaX) * ((n_[1] + kh::kTmaY - 1) / kh::kTmaY);
+      const long long xy = (long long)((n_[0] + kh::kLeanX - 1) / kh::kLeanX) * ((n_[1] + kh::kLeanY - 1) / kh::kLeanY);
       const long long fill = xy * n_[2] / (2LL * tma_slots_);
       z = int(std::max(2LL, std::min<long long>(z, fill)));
     }
     return std::min(z, n_[2]);
+  }
+
+  // T, U and W of every CPML cell brought up to date from the reduced state.
+  kh_status expand_state() {
+    if (complete_state_ || !(pml_axis_[0] || pml_axis_[1] || pml_axis_[2])) return KH_OK;
+    for (int h = 0; h < 2; ++h) {
+      if (!reduced_[h]) continue;
+      kh::launch_expand_state<T>(h == 1, base_params(h == 1), cudaStreamLegacy);
+      ++launches;
+    }
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    if (e != cudaSuccess) return fail(KH_ERR_CUDA, std::string("state expansion: ") + cudaGetErrorString(e));
+    return KH_OK;
   }
 
   kh_status device_error() override { return check_device_error(); }
@@ -2142,7 +2194,14 @@ class Sim : public SimBase {
   int xprefetch_ = 2;        // x-CPML state prefetch mode (HalfStepParams::xprefetch)
   int xpf_dist_ = 3;
   int tma_slots_ = 0;  // SMs × resident TMA-kernel CTAs per SM
-  kh::TmaMaps maps_h_, maps_e_;
+  kh::TmaMaps maps_h_, maps_e_;            // kTmaY rows (general kernel)
+  kh::TmaMaps lean_maps_h_, lean_maps_e_;  // kLeanY rows (reduced-state kernel)
+  // [E half, H half]: the reduced-state kernel takes this half's launches.  T, U
+  // and W that follow from the rest of the state are then not kept up to date.
+  bool reduced_[2] = {false, false};
+  // A material of a CPML cell changed mid-run, so W = m·T no longer holds: the
+  // general kernel carries on from the complete state until reset().
+  bool complete_state_ = false;
 
   std::vector<void*> allocs_;
   std::vector<std::pair<void*, size_t>> state_;
@@ -2290,7 +2349,7 @@ kh_status kh_debug_bounds(int64_t* count, int64_t* index, int32_t* site) {
   *site = 0;
 #ifdef KH_DEBUG_BOUNDS
   if (cudaDeviceSynchronize() != cudaSuccess) return KH_ERR_CUDA;
-  void (*readers[])(unsigned long long*, long long*, int*) = {kh::dbg_read_tma, kh::dbg_read_kernels};
+  void (*readers[])(unsigned long long*, long long*, int*) = {kh::dbg_read_tma, kh::dbg_read_kernels, kh::dbg_read_lean};
   for (auto rd : readers) {
     unsigned long long c = 0;
     long long ix = 0;

@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/khronos_gb300.h"
+#include "kh_async.cuh"
 #include "kh_cell.cuh"
 
 namespace kh {
@@ -30,70 +31,6 @@ KH_DBG_READER(dbg_read_tma)
 #endif
 
 namespace {
-
-constexpr long long kWaitLimit = 1ll << 22;
-constexpr long long kStallWaitLimit = 4096;  // the failure-detection test hook's limit
-
-__device__ __forceinline__ uint32_t smem_u32(const void* ptr) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(ptr));
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_fence_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait for the phase with parity `parity`; false after `limit` polls.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit = kWaitLimit) {
-  for (long long it = 0; it < limit; ++it)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
-
-__device__ __forceinline__ void fence_proxy_async() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
-                                            uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// L2 prefetch of one tensor-map tile (no shared memory, no completion).
-__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int x, int y, int z) {
-  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(
-                   reinterpret_cast<uint64_t>(map)),
-               "r"(x), "r"(y), "r"(z)
-               : "memory");
-}
-
-__device__ __forceinline__ void l2_prefetch(const void* ptr) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(ptr));
-}
 
 template <typename T>
 struct TmaGeom {
@@ -502,8 +439,7 @@ template <typename T>
 void launch_half_step_tma(bool h_half, const HalfStepParams<T>& p, const TmaMaps& maps, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (p.cpml) {
-    if (p.full) launch_tma_variant<T, true, true>(h_half, p, maps, st);
-    else launch_tma_variant<T, true, false>(h_half, p, maps, st);
+    launch_tma_variant<T, true, true>(h_half, p, maps, st);
   } else {
     if (p.full) launch_tma_variant<T, false, true>(h_half, p, maps, st);
     else launch_tma_variant<T, false, false>(h_half, p, maps, st);
@@ -520,29 +456,16 @@ template <typename T>
 int prepare_tma_kernels() {
   int e = 0;
   e |= set_smem_attr<T, true, true, true>();
-  e |= set_smem_attr<T, true, true, false>();
   e |= set_smem_attr<T, true, false, true>();
   e |= set_smem_attr<T, true, false, false>();
   e |= set_smem_attr<T, false, true, true>();
-  e |= set_smem_attr<T, false, true, false>();
   e |= set_smem_attr<T, false, false, true>();
   e |= set_smem_attr<T, false, false, false>();
   if constexpr (sizeof(T) == 4) {
-    e |= set_smem_attr<T, true, true, false, true>();
     e |= set_smem_attr<T, true, false, false, true>();
-    e |= set_smem_attr<T, false, true, false, true>();
     e |= set_smem_attr<T, false, false, false, true>();
   }
   return e;
-}
-
-template <typename T>
-int tma_resident_ctas() {
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, half_step_tma_kernel<T, true, true, false>, 32 * kTmaY,
-                                                    TmaGeom<T>::SMEM) != cudaSuccess)
-    return 1;
-  return n > 0 ? n : 1;
 }
 
 template size_t tma_smem_bytes<float>();
@@ -551,7 +474,5 @@ template void launch_half_step_tma<float>(bool, const HalfStepParams<float>&, co
 template void launch_half_step_tma<double>(bool, const HalfStepParams<double>&, const TmaMaps&, void*);
 template int prepare_tma_kernels<float>();
 template int prepare_tma_kernels<double>();
-template int tma_resident_ctas<float>();
-template int tma_resident_ctas<double>();
 
 }  // namespace kh
