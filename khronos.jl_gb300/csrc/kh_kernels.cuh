@@ -394,11 +394,15 @@ struct DispFixParams {
 // (update_dft_monitor!, Monitors.jl:361-379, for all monitors updated at this
 // step): item t of monitor m (t < ncell·nf, cell fastest) is (cell, f).
 constexpr int kMaxDftBatch = 16;
+constexpr int kDftThreads = 256;
+constexpr int kDftFreqs = 8;  // frequencies of a block of a large launch
 template <typename T>
 struct DftBatchParams {
   int n;                             // monitors in this launch
   long long pitch, plane, origin, total;
-  long long first[kMaxDftBatch + 1]; // prefix sums of the monitors' items
+  // set by launch_dft_batch: prefix sums of the monitors' blocks, frequencies of a block
+  unsigned first[kMaxDftBatch + 1];
+  int freqs;
   struct Mon {
     const T* field;
     int start[3], dims[3];

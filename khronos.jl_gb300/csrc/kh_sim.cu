@@ -1832,7 +1832,6 @@ class Sim : public SimBase {
       bp.plane = plane_;
       bp.origin = origin_;
       bp.total = total_;
-      bp.first[0] = 0;
       for (size_t q = b0; q < dms.size() && bp.n < kh::kMaxDftBatch; ++q) {
         const Mon& m = mons_[dms[q].first];
         auto& M = bp.mon[bp.n];
@@ -1845,7 +1844,6 @@ class Sim : public SimBase {
         M.phase = dtab + dms[q].second;
         M.F = m.F;
         M.comp = m.C;
-        bp.first[bp.n + 1] = bp.first[bp.n] + (long long)m.ncell * m.nf;
         ++bp.n;
       }
       kh::launch_dft_batch<T>(bp, st);
