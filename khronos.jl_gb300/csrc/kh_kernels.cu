@@ -402,19 +402,21 @@ void launch_source_fix(const SourceFixParams<T>& p, void* stream) {
 // warp per entry of the row-segment list (32·kVN cells).  A segment without
 // pole cells needs no class words: its lanes load the pair of E vectors and
 // χ3 values of their two cells at once and correct the cells with χ3 ≠ 0
-// (the cells the LEAN launch left uncorrected).  Pole segments go cell by
-// cell through the class words.
+// (the cells the LEAN launch left uncorrected).  Pole segments go through the
+// class words, pair by pair (256³ with a χ3 slab and two poles' spheres: 57 to 52 µs
+// a launch against cell by cell; reading σ first to leave out absent poles puts
+// a round trip before the rest: 58).
 template <typename T>
 __global__ void disp_fix_kernel(const DispFixParams<T> p) {
   static_assert(kVN == 2, "paired loads of the χ3 path");
   const long long w = (long long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   if (w >= p.n_list) return;  // warp-uniform
   const uint32_t ent = p.list[w];
-  const long long seg = ent & 0x7fffffffu;
-  const int xb = int(seg % p.nxb);
-  const long long r = seg / p.nxb;
-  const int j = int(r % p.ny);
-  const int k = int(r / p.ny);
+  const unsigned seg = ent & 0x7fffffffu;
+  const unsigned r = seg / unsigned(p.nxb);
+  const int xb = int(seg - r * unsigned(p.nxb));
+  const int k = int(r / unsigned(p.ny));
+  const int j = int(r - unsigned(k) * unsigned(p.ny));
   const int lane = threadIdx.x & 31;
   const int i0 = xb * 32 * kVN + lane * kVN;
   const long long q0 = p.origin + (long long)k * p.plane + (long long)j * p.pitch + i0;
@@ -447,48 +449,85 @@ __global__ void disp_fix_kernel(const DispFixParams<T> p) {
       return;
     }
   }
-#pragma unroll 1
-  for (int v = 0; v < kVN; ++v) {
-    const int i = i0 + v;
-    if (i >= p.nx) continue;
-    const long long q = q0 + v;
-    if (!KH_IN(q, p.total, 3040)) continue;
-    const uint32_t cls = p.cell_class[q];
-    if (!(cls & (kHasChi3 | kHasPole))) continue;
-    T O[3];
-    if (cls & kHasPole) {
+  // Both cells of a lane at once: every array is read as a pair (the row padding
+  // makes the second one readable past an odd row's end), so a lane's loads of a
+  // stage are in flight together.
+  if (i0 >= p.nx || !(KH_IN(q0, p.total, 3040) && KH_IN(q0 + 1, p.total, 3040))) return;
+  using V2 = typename VT<T, 2>::V;
+  const bool two = i0 + 1 < p.nx;
+  const uint2 cl = *reinterpret_cast<const uint2*>(p.cell_class + q0);
+  const uint32_t cls[2] = {cl.x, two ? cl.y : 0u};
+  if (!((cls[0] | cls[1]) & (kHasChi3 | kHasPole))) return;
+  auto ld = [&](const T* a, T (&x)[2]) {
+    const V2 w = *reinterpret_cast<const V2*>(a + q0);
+    x[0] = w.x;
+    x[1] = w.y;
+  };
+  auto st = [&](T* a, const T (&x)[2]) {
+    if (two) {
+      V2 w;
+      w.x = x[0];
+      w.y = x[1];
+      *reinterpret_cast<V2*>(a + q0) = w;
+    } else {
+      a[q0] = x[0];
+    }
+  };
+  const bool pole[2] = {(cls[0] & kHasPole) != 0, (cls[1] & kHasPole) != 0};
+  T O[3][2], c3[2] = {T(0), T(0)};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) ld(p.E[c], O[c]);
+  if (p.chi3) ld(p.chi3, c3);
+  if (pole[0] || pole[1]) {
+    T D[3][2], m[3][2], Ptot[3][2] = {};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      ld(p.D[c], D[c]);
+      if (p.m_inv[c]) ld(p.m_inv[c], m[c]);
+      else m[c][0] = m[c][1] = p.m_scalar;
+    }
+    for (int pp = 0; pp < p.npoles; ++pp) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        T P[2];
+        ld(p.poles[pp].P[c], P);
+        Ptot[c][0] += P[0];
+        Ptot[c][1] += P[1];
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      if (!pole[v]) continue;
       // E = ε⁻¹·(D + S − Σ P) (update_field_generic: net = T; net += S; net -= P)
       T S[3] = {T(0), T(0), T(0)};
       bool hasS[3] = {false, false, false};
-      if (p.sources_active && (cls & kHasSrcE)) {
-        const int slot = int(cls >> kSlotShift);
+      if (p.sources_active && (cls[v] & kHasSrcE)) {
+        const int slot = int(cls[v] >> kSlotShift);
         if (KH_IN(slot + 1, p.n_slots + 1, 3041)) {
           for (int e = p.slot_off[slot]; e < p.slot_off[slot + 1]; ++e) {
             if (!KH_IN(e, p.n_ent, 3042) || !KH_IN(p.ent_src[e], p.n_src, 3043)) continue;
             const int c = p.ent_comp[e];
             const Cplx<T> am = p.ent_amp[e];
             const Cplx<T> fv = p.f_now[p.ent_src[e]];
-            const T v = fv.re * am.re - fv.im * am.im;  // real(f(t) · amplitude)
-            if (c >= 0 && c < 3) {
-              S[c] += v;
-              hasS[c] = true;
-            }
+            const T x = fv.re * am.re - fv.im * am.im;  // real(f(t) · amplitude)
+#pragma unroll
+            for (int o = 0; o < 3; ++o)
+              if (c == o) {
+                S[o] += x;
+                hasS[o] = true;
+              }
           }
         }
       }
-      T Ptot[3] = {T(0), T(0), T(0)};
-      for (int pp = 0; pp < p.npoles; ++pp) {
-        Ptot[0] += p.poles[pp].P[0][q];
-        Ptot[1] += p.poles[pp].P[1][q];
-        Ptot[2] += p.poles[pp].P[2][q];
-      }
+      const int i = i0 + v;
+      const long long q = q0 + v;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        T net = p.D[c][q];
+        T net = D[c][v];
         if (hasS[c]) net += S[c];
-        net -= Ptot[c];
-        const T m = p.m_inv[c] ? p.m_inv[c][q] : p.m_scalar;
-        O[c] = m * net;
+        net -= Ptot[c][v];
+        const T e0 = O[c][v];
+        O[c][v] = m[c][v] * net;
         // in the CPML of its own axis the cell's E comes out of the W stage
         // (update_field_generic, Helpers.jl:333-339): E = E' + op·(W_new − W')
         // on top of the W' and E' that the LEAN launch (or the source kernel)
@@ -500,49 +539,55 @@ __global__ void disp_fix_kernel(const DispFixParams<T> p) {
             const AxisCoef<T> ao = p.ax[c][idx];
             if (ao.s != T(0)) {
               const T wl = p.W[c][q];
-              const T wn = m * net;
+              const T wn = m[c][v] * net;
               p.W[c][q] = wn;
-              O[c] = p.E[c][q] + ao.op * (wn - wl);
+              O[c][v] = e0 + ao.op * (wn - wl);
             }
           }
         }
       }
-    } else {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) O[c] = p.E[c][q];
     }
-    // χ3 Kerr correction (Dispersive.jl:127-147)
-    if (cls & kHasChi3) {
-      const T c3 = p.chi3[q];
-      if (c3 != T(0)) {
-        const T esq = (O[0] * O[0] + O[1] * O[1]) + O[2] * O[2];
-        const T corr = T(1) / (T(1) + c3 * esq);
-        O[0] = O[0] * corr;
-        O[1] = O[1] * corr;
-        O[2] = O[2] * corr;
-      }
-    }
-    // ADE poles with E^{n+1} (Dispersive.jl:25-88)
-    if (cls & kHasPole) {
-      for (int pp = 0; pp < p.npoles; ++pp) {
-        const PoleParams<T>& P = p.poles[pp];
-        const T s = P.sigma[q];
-        if (s == T(0)) continue;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const T px = P.P[c][q];
-          const T pprev = P.Pprev[c][q];
-          T pn;
-          if (P.is_drude) pn = P.gamma1_inv * ((T(2) * px - P.gamma1 * pprev) + (P.drive * s) * O[c]);
-          else pn = P.gamma1_inv * ((P.coeff_p * px - P.gamma1 * pprev) + (P.drive * s) * O[c]);
-          P.P[c][q] = pn;
-          P.Pprev[c][q] = px;
-        }
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) p.E[c][q] = O[c];
   }
+#pragma unroll
+  for (int v = 0; v < 2; ++v) {
+    // χ3 Kerr correction (Dispersive.jl:127-147)
+    if ((cls[v] & kHasChi3) && c3[v] != T(0)) {
+      const T esq = (O[0][v] * O[0][v] + O[1][v] * O[1][v]) + O[2][v] * O[2][v];
+      const T corr = T(1) / (T(1) + c3[v] * esq);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) O[c][v] = O[c][v] * corr;
+    }
+  }
+  // ADE poles with E^{n+1} (Dispersive.jl:25-88)
+  if (pole[0] || pole[1]) {
+    for (int pp = 0; pp < p.npoles; ++pp) {
+      const PoleParams<T>& P = p.poles[pp];
+      T s[2], px[3][2], pv[3][2];
+      ld(P.sigma, s);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        ld(P.P[c], px[c]);
+        ld(P.Pprev[c], pv[c]);
+      }
+      const bool act[2] = {pole[0] && s[0] != T(0), pole[1] && s[1] != T(0)};
+      if (!(act[0] || act[1])) continue;
+      const T cp = P.is_drude ? T(2) : P.coeff_p;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          if (!act[v]) continue;
+          const T pn = P.gamma1_inv * ((cp * px[c][v] - P.gamma1 * pv[c][v]) + (P.drive * s[v]) * O[c][v]);
+          pv[c][v] = px[c][v];
+          px[c][v] = pn;
+        }
+        st(P.P[c], px[c]);
+        st(P.Pprev[c], pv[c]);
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) st(p.E[c], O[c]);
 }
 
 template <typename T>
