@@ -85,6 +85,7 @@ __device__ __forceinline__ bool dbg_in(long long idx, long long n, int site) {
 void dbg_read_tma(unsigned long long* count, long long* index, int* site);
 void dbg_read_kernels(unsigned long long* count, long long* index, int* site);
 void dbg_read_lean(unsigned long long* count, long long* index, int* site);
+void dbg_read_fused(unsigned long long* count, long long* index, int* site);
 #else
 #define KH_IN(idx, n, site) true
 #endif
@@ -244,6 +245,47 @@ struct alignas(128) TmaMaps {
   CUtensorMap u[3];
   CUtensorMap w[3];
 };
+
+// Whole-step kernel (kh_fused.cu): 8 rows of threads (a halo row and 7 owned),
+// ring stages, resident CTAs per SM, owned columns at most.  Two stages are in use
+// while a plane is computed; with a fourth fewer CTAs fit (216×200×168 with per-voxel
+// ε, 100 steps: 2 / 3 / 4 stages 9.87 / 8.56 / 8.71 ms).
+constexpr int kFusedRows = 8;
+constexpr int kFusedStages = 3;
+constexpr int kFusedMinBlocks = 4;
+constexpr int kFusedW = kTmaX - 4;
+
+// One step of a grid without CPML from one set of E and H into the other.
+template <typename T>
+struct FusedParams {
+  int nx, ny, nz;
+  long long pitch, plane, origin, total;
+  int nxb;
+  int zplanes;
+  int tile_w;  // owned columns of a tile: a multiple of 4, at most kFusedW
+  int pervox_eps;
+  T cd[3];
+  T mu_scalar, eps_scalar;
+  T *En[3], *Hn[3];
+  T* D[3];  // D state of special cells, in place
+  const uint64_t* tile_bits;
+  long long n_tile_words;
+  const uint32_t* cell_class;
+  int* err;
+};
+
+// Boxes: E (kTmaX + 16 bytes) × (kFusedRows + 1), H kTmaX × kFusedRows,
+// ε⁻¹ kTmaX × (kFusedRows - 1).
+struct alignas(128) FusedMaps {
+  CUtensorMap e[3], h[3], m[3];
+};
+
+template <typename T>
+void launch_step_fused(const FusedParams<T>& p, const FusedMaps& maps, void* stream);
+template <typename T>
+int prepare_fused_kernels();
+template <typename T>
+int fused_resident_ctas();
 
 template <typename T>
 size_t tma_smem_bytes();

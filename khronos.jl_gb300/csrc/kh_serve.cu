@@ -105,6 +105,7 @@ struct kh_server {
       ++resident;
       r->state = KH_REQ_ADMITTED;
       lk.unlock();
+      r->sim->impl->no_second_set();  // the budget admits what the estimate says
       const kh_status st = r->sim->impl->prepare();
       const int64_t actual = r->sim->impl->device_bytes();
       lk.lock();

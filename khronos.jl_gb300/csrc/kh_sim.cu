@@ -839,6 +839,7 @@ class Sim : public SimBase {
       reduced_[0] = !(msigd_[0] || msigd_[1] || msigd_[2]) && (!dispersive || disp_fix_);
       reduced_[1] = !(msigb_[0] || msigb_[1] || msigb_[2]);
     }
+    KH_TRY(prepare_fused());
     prepared_ = true;
     return KH_OK;
 #undef KH_TRY
@@ -865,6 +866,7 @@ class Sim : public SimBase {
   int step_alignment() const override { return align_; }
   int64_t graph_replays() const override { return graph_replays_; }
 
+  void no_second_set() override { second_set_ok_ = false; }
   int64_t timestep() const override { return timestep_; }
   int sources_active() const override { return sources_active_ ? 1 : 0; }
   bool is_prepared() const override { return prepared_; }
@@ -1605,8 +1607,42 @@ class Sim : public SimBase {
     const kh::WrapParams<T> wh = wrap_params(true), we = wrap_params(false);
     kh::SourceFixParams<T> fh = fix_params(true), fe = fix_params(false);
     kh::DispFixParams<T> dfix = disp_params(pe);
+    // what follows the E update of a step, on the current set of fields
+    auto after_e = [&](const StepPlan& P, cudaStream_t st) {
+      if (P.sa && has_src_[0] && !pe.full) {
+        fe.f_now = dtab + P.fE;
+        for (int c = 0; c < 3; ++c) fe.O[c] = cur_E(c);
+        kh::launch_source_fix<T>(fe, st);
+        ++launches;
+      }
+      if (disp_fix_ && !pe.full) {
+        dfix.sources_active = P.sa ? 1 : 0;
+        dfix.f_now = dtab + P.fE;
+        for (int c = 0; c < 3; ++c) dfix.E[c] = cur_E(c);
+        kh::launch_disp_fix<T>(dfix, st);
+        ++launches;
+      }
+    };
+    const bool whole = fused_ && !timing && !complete_state_;
     auto issue_all = [&](cudaStream_t st) {
     for (int s = 0; s < nb; ++s) {
+      // two whole steps, into the second set and back
+      if (whole && s + 1 < nb) {
+        pe.full = 0;
+        for (int q = 0; q < 2; ++q) {
+          const StepPlan& P = plan[s + q];
+          launch_fused(q, st);
+          cur_ = 1 - q;
+          after_e(P, st);
+          std::vector<std::pair<int, size_t>> dms(P.dftH);
+          dms.insert(dms.end(), P.dftE.begin(), P.dftE.end());
+          launch_dfts(dms, dtab, st);
+          record_histories(true, timestep_ + s + q, st);
+          record_histories(false, timestep_ + s + q, st);
+        }
+        ++s;
+        continue;
+      }
       const StepPlan& P = plan[s];
       ph.sources_active = P.sa ? 1 : 0;
       ph.f_now = dtab + P.fH;
@@ -1638,17 +1674,7 @@ class Sim : public SimBase {
       else if (use_tma_) kh::launch_half_step_tma<T>(false, pe, maps_e_, st);
       else kh::launch_half_step<T>(false, pe, st);
       ++launches;
-      if (src_e && !pe.full) {
-        fe.f_now = dtab + P.fE;
-        kh::launch_source_fix<T>(fe, st);
-        ++launches;
-      }
-      if (disp_fix_ && !pe.full) {
-        dfix.sources_active = P.sa ? 1 : 0;
-        dfix.f_now = dtab + P.fE;
-        kh::launch_disp_fix<T>(dfix, st);
-        ++launches;
-      }
+      after_e(P, st);
       if (d_.periodic) {
         kh::launch_wrap<T>(we, st);
         ++launches;
@@ -1762,7 +1788,7 @@ class Sim : public SimBase {
     for (auto& h : hists_) {
       if ((h.comp >= 3) != h_half || ts >= h.cap) continue;
       kh::RecordParams<T> p;
-      p.field = h.comp < 3 ? E_[h.comp] : H_[h.comp - 3];
+      p.field = h.comp < 3 ? cur_E(h.comp) : cur_H(h.comp - 3);
       p.pitch = pitch_;
       p.plane = plane_;
       p.origin = origin_;
@@ -1835,7 +1861,7 @@ class Sim : public SimBase {
       for (size_t q = b0; q < dms.size() && bp.n < kh::kMaxDftBatch; ++q) {
         const Mon& m = mons_[dms[q].first];
         auto& M = bp.mon[bp.n];
-        M.field = m.comp < 3 ? E_[m.comp] : H_[m.comp - 3];
+        M.field = m.comp < 3 ? cur_E(m.comp) : cur_H(m.comp - 3);
         for (int a = 0; a < 3; ++a) {
           M.start[a] = m.start[a];
           M.dims[a] = m.dims[a];
@@ -1854,7 +1880,7 @@ class Sim : public SimBase {
   void launch_dft_for(int mi, const Cplx<T>* phase, cudaStream_t stream) {
     const Mon& m = mons_[mi];
     kh::DftParams<T> p;
-    p.field = m.comp < 3 ? E_[m.comp] : H_[m.comp - 3];
+    p.field = m.comp < 3 ? cur_E(m.comp) : cur_H(m.comp - 3);
     p.pitch = pitch_;
     p.plane = plane_;
     p.origin = origin_;
@@ -1903,10 +1929,13 @@ class Sim : public SimBase {
     if (!attr_done[dev]) {
       if (kh::prepare_tma_kernels<T>() != 0 || kh::prepare_lean_kernels<T>() != 0)
         return fail(KH_ERR_CUDA, "cudaFuncSetAttribute on the TMA half-step kernels failed");
+      if (sizeof(T) == 4 && kh::prepare_fused_kernels<float>() != 0)
+        return fail(KH_ERR_CUDA, "cudaFuncSetAttribute on the whole-step kernels failed");
       attr_done[dev] = true;
     }
     int sms = 0;
     KH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (sizeof(T) == 4) fused_slots_ = sms * kh::fused_resident_ctas<float>();
     tma_slots_ = sms * kh::lean_resident_ctas<T>();
     const int hx = 16 / int(sizeof(T));
     struct MapSet {
@@ -1956,6 +1985,102 @@ class Sim : public SimBase {
     }
     return std::min(z, n_[2]);
   }
+
+  // Whole-step launches on grids without CPML where nothing comes between the
+  // halves (periodic wraps, H sources).  With CPML they lose: the tiles that meet
+  // it are bound by instructions, and the halo adds a third of them (320×192×128:
+  // 16.4 ms for 96 steps in half-steps, 18.8 in whole steps).  FP64 is bound by
+  // arithmetic and keeps the half-steps too.  The second set of arrays is taken
+  // only while it is a small part of the free memory.  KHRONOS_GB300_FUSED=0 turns
+  // them off.
+  kh_status prepare_fused() {
+    fused_ = false;
+    if constexpr (sizeof(T) == 4) {
+      const char* fv = std::getenv("KHRONOS_GB300_FUSED");
+      if (!second_set_ok_ || !reduced_[0] || !reduced_[1] || pml_axis_[0] || pml_axis_[1] || pml_axis_[2] ||
+          d_.periodic || has_src_[1] || mu_[0] || stall_tx_ || (fv && std::string(fv) == "0"))
+        return KH_OK;
+      const size_t field = size_t(total_ + pitch_) * sizeof(T);
+      size_t free_b = 0, all_b = 0;
+      KH_CUDA(cudaMemGetInfo(&free_b, &all_b));
+      if (6 * field > free_b / 16) return KH_OK;
+      for (int c = 0; c < 6; ++c)
+        if (alloc_raw(field, (void**)(c < 3 ? &E2_[c] : &H2_[c - 3]), false) != KH_OK) {
+          cudaGetLastError();  // somebody took the memory: half-steps
+          err.clear();
+          return KH_OK;
+        }
+      for (int h = 0; h < 2; ++h) {
+        kh::FusedMaps& fm = fused_maps_[h];
+        std::memset(&fm, 0, sizeof(fm));
+        const cuuint32_t hx = 16 / sizeof(T);
+        const cuuint32_t be[3] = {cuuint32_t(kh::kTmaX) + hx, cuuint32_t(kh::kFusedRows + 1), 1};
+        const cuuint32_t bh[3] = {cuuint32_t(kh::kTmaX), cuuint32_t(kh::kFusedRows), 1};
+        const cuuint32_t bm[3] = {cuuint32_t(kh::kTmaX), cuuint32_t(kh::kFusedRows - 1), 1};
+        for (int c = 0; c < 3; ++c) {
+          kh_status st;
+          if ((st = encode_map(&fm.e[c], h ? E2_[c] : E_[c], be)) != KH_OK) return st;
+          if ((st = encode_map(&fm.h[c], h ? H2_[c] : H_[c], bh)) != KH_OK) return st;
+          if (eps_[c] && (st = encode_map(&fm.m[c], eps_[c], bm)) != KH_OK) return st;
+        }
+      }
+      // as few column tiles as fit, of equal width; whole 32-byte sectors where
+      // that does not cost a tile
+      const int nt = (n_[0] + kh::kFusedW - 1) / kh::kFusedW;
+      const int even = (n_[0] + nt - 1) / nt;
+      fused_w_ = (even + 7) / 8 * 8;
+      if (fused_w_ > kh::kFusedW) fused_w_ = (even + 3) / 4 * 4;
+      const long long xy = (long long)nt * ((n_[1] + kh::kFusedRows - 2) / (kh::kFusedRows - 1));
+      // Planes per CTA: the fewest (from 2) whose CTAs are all resident at once, at
+      // most 16.  Fewer read the halo planes more often, more leave SMs idle (64³:
+      // 2.33 / 2.00 / 2.10 / 2.43 ms for 200 steps at 2 / 3 / 4 / 8 planes, in
+      // half-steps 2.14; 100×90×110: 3.53 / 3.40 / 3.02 / 3.16 at 3 / 5 / 8 / 12, 4.23;
+      // 216×200×168: 9.12 / 8.71 / 8.53 / 8.45 at 4 / 8 / 16 / 24, 11.18).
+      long long z = 2;
+      while (z < 16 && xy * ((n_[2] + z - 1) / z) > fused_slots_) ++z;
+      if (const char* zv = std::getenv("KHRONOS_GB300_ZPLANES")) z = std::max(1, std::atoi(zv));
+      fused_zplanes_ = int(std::min<long long>(z, n_[2]));
+      KH_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the zeroing of the second set
+      fused_ = true;
+    }
+    return KH_OK;
+  }
+
+  // One step from set `from` into the other.
+  void launch_fused(int from, cudaStream_t st) {
+    if constexpr (sizeof(T) == 4) {
+      kh::FusedParams<T> p;
+      std::memset(&p, 0, sizeof(p));
+      p.nx = n_[0];
+      p.ny = n_[1];
+      p.nz = n_[2];
+      p.pitch = pitch_;
+      p.plane = plane_;
+      p.origin = origin_;
+      p.total = total_;
+      p.nxb = nxb_;
+      p.zplanes = fused_zplanes_;
+      p.tile_w = fused_w_;
+      p.pervox_eps = eps_[0] != nullptr;
+      p.mu_scalar = T(d_.mu_inv);
+      p.eps_scalar = T(d_.eps_inv);
+      for (int c = 0; c < 3; ++c) {
+        p.cd[c] = dt_ * (T(1) / delta_[c]);
+        p.En[c] = from ? E_[c] : E2_[c];
+        p.Hn[c] = from ? H_[c] : H2_[c];
+        p.D[c] = D_[c];
+      }
+      p.tile_bits = tbits_e_;
+      p.n_tile_words = tbits_e_ ? (long long)((n_[2] + 63) / 64) * n_[1] * nxb_ : 0;
+      p.cell_class = cls_;
+      p.err = err_dev_;
+      kh::launch_step_fused<T>(p, fused_maps_[from], st);
+      ++launches;
+    }
+  }
+
+  T* cur_E(int c) const { return cur_ ? E2_[c] : E_[c]; }
+  T* cur_H(int c) const { return cur_ ? H2_[c] : H_[c]; }
 
   // T, U and W of every CPML cell brought up to date from the reduced state.
   kh_status expand_state() {
@@ -2191,6 +2316,7 @@ class Sim : public SimBase {
   int zplanes_ = 10;
   int xprefetch_ = 2;        // x-CPML state prefetch mode (HalfStepParams::xprefetch)
   int xpf_dist_ = 3;
+  int fused_slots_ = 1;  // SMs × resident whole-step CTAs per SM
   int tma_slots_ = 0;  // SMs × resident TMA-kernel CTAs per SM
   kh::TmaMaps maps_h_, maps_e_;            // kTmaY rows (general kernel)
   kh::TmaMaps lean_maps_h_, lean_maps_e_;  // kLeanY rows (reduced-state kernel)
@@ -2200,6 +2326,14 @@ class Sim : public SimBase {
   // A material of a CPML cell changed mid-run, so W = m·T no longer holds: the
   // general kernel carries on from the complete state until reset().
   bool complete_state_ = false;
+  // Whole-step launches (kh_fused.cu): the second set of E and H, the tensor maps
+  // from set 0 into 1 and back, and the set that holds the current fields (1 only
+  // between the two steps of a pair).
+  bool second_set_ok_ = true, fused_ = false;
+  T *E2_[3] = {}, *H2_[3] = {};
+  kh::FusedMaps fused_maps_[2];
+  int fused_zplanes_ = 1, fused_w_ = kh::kFusedW;
+  int cur_ = 0;
 
   std::vector<void*> allocs_;
   std::vector<std::pair<void*, size_t>> state_;
@@ -2347,7 +2481,8 @@ kh_status kh_debug_bounds(int64_t* count, int64_t* index, int32_t* site) {
   *site = 0;
 #ifdef KH_DEBUG_BOUNDS
   if (cudaDeviceSynchronize() != cudaSuccess) return KH_ERR_CUDA;
-  void (*readers[])(unsigned long long*, long long*, int*) = {kh::dbg_read_tma, kh::dbg_read_kernels, kh::dbg_read_lean};
+  void (*readers[])(unsigned long long*, long long*, int*) = {kh::dbg_read_tma, kh::dbg_read_kernels, kh::dbg_read_lean,
+                                                               kh::dbg_read_fused};
   for (auto rd : readers) {
     unsigned long long c = 0;
     long long ix = 0;

@@ -57,6 +57,8 @@ struct SimBase {
   virtual kh_status add_monitor(int comp, const int32_t* st, const int32_t* dm, int nf,
                                 const double* f, int dec, int32_t* id) = 0;
   virtual kh_status prepare() = 0;
+  // Before prepare: keep to the arrays that estimate_bytes() counts.
+  virtual void no_second_set() = 0;
   virtual bool is_prepared() const = 0;
   virtual kh_status step(int64_t n, cudaStream_t s) = 0;
   virtual int64_t timestep() const = 0;
