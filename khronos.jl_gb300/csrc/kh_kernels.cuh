@@ -228,6 +228,7 @@ constexpr int kLeanY = 4;
 constexpr int kLeanVN = 2;
 constexpr int kLeanStages = 3;
 constexpr int kLeanXpf = 3;
+constexpr int kLeanZ = 64;  // z planes of a CTA at most
 template <typename T>
 constexpr int kLeanMinBlocks = sizeof(T) == 4 ? 6 : 3;
 

@@ -43,7 +43,7 @@ struct LeanGeom {
   static constexpr int O_ELEMS = kLeanX * kLeanY;
   static constexpr int STAGE = 3 * A_ELEMS + (PV ? 6 : 3) * O_ELEMS;  // A0..2, O0..2(, m0..2)
   static constexpr size_t SMEM =
-      size_t(kLeanStages) * STAGE * sizeof(T) + kLeanX * sizeof(AxisCoef<T>) + kLeanStages * sizeof(uint64_t);
+      size_t(kLeanStages) * STAGE * sizeof(T) + (kLeanX + kLeanZ) * sizeof(AxisCoef<T>) + kLeanStages * sizeof(uint64_t);
 };
 
 }  // namespace
@@ -55,13 +55,19 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
     half_step_lean_kernel(const __grid_constant__ HalfStepParams<T> p, const __grid_constant__ TmaMaps maps) {
   using G = LeanGeom<T, PV>;
   constexpr int VN = kLeanVN;
+  // Rows in update_row's branch-free forms, except in FP32 with per-voxel m⁻¹, where
+  // their longer live ranges spill at six CTAs per SM (320×192×128, 96 steps: 15.96 ms
+  // with update_cells in both halves, 15.37 with this choice, 15.73 with update_row in
+  // both; FP64 240×144×96, where a branch costs both sides' arithmetic, 17.9 to 13.0).
+  constexpr bool kRow = sizeof(T) == 8 || !PV;
   constexpr int LPR = kLeanX / VN;  // lanes per tile row
   using PK = Pack<T, VN>;
   constexpr int s = H ? 1 : -1;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   T* stages = reinterpret_cast<T*>(smem_raw);
   AxisCoef<T>* xtab = reinterpret_cast<AxisCoef<T>*>(stages + kLeanStages * G::STAGE);  // per tile column: a, b, om, op
-  uint64_t* bars = reinterpret_cast<uint64_t*>(xtab + kLeanX);
+  AxisCoef<T>* ztab = xtab + kLeanX;                                                    // per plane of the chunk
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ztab + kLeanZ);
 
   const int tid = threadIdx.x;
   const int col = (tid % LPR) * VN;
@@ -90,6 +96,12 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
       const bool f = i < p.nx && (i < p.pml_lo[0] || i >= p.nx - p.pml_hi[0]);
       const RedAxis<T> r = red_axis<T>(f && KH_IN(i, p.nx, 2120) ? p.ax[0][i] : AxisCoef<T>{}, f);
       xtab[c] = {r.a, r.b, r.om, r.op};
+    }
+  if (k0 < p.pml_lo[2] || k1 > p.nz - p.pml_hi[2])
+    for (int c = tid; c < N; c += kLeanThreads) {
+      const bool f = k0 + c < p.pml_lo[2] || k0 + c >= p.nz - p.pml_hi[2];
+      const RedAxis<T> r = red_axis<T>(f && KH_IN(k0 + c, p.nz, 2112) ? p.ax[2][k0 + c] : AxisCoef<T>{}, f);
+      ztab[c] = {r.a, r.b, r.om, r.op};
     }
   __syncthreads();
 
@@ -188,7 +200,7 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
     // auxiliaries: T in the own-axis CPML, U in those of both other axes; rows
     // with special cells take all of them
     Cells<T, VN> t, u;
-    AxisCoef<T> cz{};
+    if constexpr (kRow) t = u = Cells<T, VN>{};
     if (!plain && lane_ok) {
       if (anyfx || tf) t.c[0] = get(p.Ts[0], 2104);
       if (fy || tf) t.c[1] = get(p.Ts[1], 2105);
@@ -196,7 +208,6 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
       if (fy && (fz || tf)) u.c[0] = get(p.U[0], 2107);
       if (fz && (anyfx || tf)) u.c[1] = get(p.U[1], 2108);
       if (anyfx && (fy || tf)) u.c[2] = get(p.U[2], 2109);
-      if (fz && KH_IN(k, p.nz, 2112)) cz = p.ax[2][k];
       if (anyfx && n + kLeanXpf < N) {
         const long long qp = q + kLeanXpf * step;
         if (KH_IN(qp + VN - 1, p.total, 2113)) {
@@ -243,34 +254,55 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
       }
       nb0 = c0;
       nb1 = c1;
-      if (plain) {
+      const AxisCoef<T> zt = ztab[k - k0];  // read where fz
+      bool sp[VN], anysp = false;
+      if (tf) {
+        constexpr uint32_t kSp = H ? kSpecialH : kSpecialE;
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-          for (int v = 0; v < VN; ++v) O.c[c].v[v] = fma_rn(m.c[c].v[v], K.c[c].v[v], O.c[c].v[v]);
+        for (int v = 0; v < VN; ++v) {
+          sp[v] = x0 + v < p.nx && KH_IN(q + v, p.total, 2110) && (p.cell_class[q + v] & kSp) != 0;
+          anysp |= sp[v];
+        }
+      }
+      if (anysp) {
+        Cells<T, VN> w;
+        if (anyfx) w.c[0] = get(p.W[0], 2128);
+        if (fy) w.c[1] = get(p.W[1], 2129);
+        if (fz) w.c[2] = get(p.W[2], 2119);
+        RedAxis<T> rz{false, T(1), T(1), T(1), T(1)};
+        if (fz) rz = {true, zt.s, zt.om, zt.ir, zt.op};
+        update_special_cells<T, VN>(sp, fxv, p.ax[0] + x0, p.ax[1] + j, fz ? p.ax[2][k].s : T(0), xtab + col, ry, rz, K,
+                                    m, O, t, u, w);
+        if (anyfx) put(p.W[0] + q, w.c[0], 2131);
+        if (fy) put(p.W[1] + q, w.c[1], 2132);
+        if (fz) put(p.W[2] + q, w.c[2], 2133);
       } else {
-        const RedAxis<T> rz = red_axis<T>(cz, fz);
-        bool sp[VN], anysp = false;
-        if (tf) {
-          constexpr uint32_t kSp = H ? kSpecialH : kSpecialE;
+        const AxisCoef<T>* xt = xtab + col;
+        if constexpr (kRow) {
+          switch ((tfx ? 1 : 0) | (fy ? 2 : 0) | (fz ? 4 : 0)) {
+            case 0: update_row<false, false, false, T, VN>(fxv, xt, ry, zt, K, m, O, t, u); break;
+            case 1: update_row<true, false, false, T, VN>(fxv, xt, ry, zt, K, m, O, t, u); break;
+            case 2: update_row<false, true, false, T, VN>(fxv, xt, ry, zt, K, m, O, t, u); break;
+            case 3: update_row<true, true, false, T, VN>(fxv, xt, ry, zt, K, m, O, t, u); break;
+            case 4: update_row<false, false, true, T, VN>(fxv, xt, ry, zt, K, m, O, t, u); break;
+            case 5: update_row<true, false, true, T, VN>(fxv, xt, ry, zt, K, m, O, t, u); break;
+            case 6: update_row<false, true, true, T, VN>(fxv, xt, ry, zt, K, m, O, t, u); break;
+            case 7: update_row<true, true, true, T, VN>(fxv, xt, ry, zt, K, m, O, t, u); break;
+          }
+        } else {
+          RedAxis<T> rz{false, T(1), T(1), T(1), T(1)};
+          if (fz) rz = {true, zt.s, zt.om, zt.ir, zt.op};
+          if (plain) {
 #pragma unroll
-          for (int v = 0; v < VN; ++v) {
-            sp[v] = x0 + v < p.nx && KH_IN(q + v, p.total, 2110) && (p.cell_class[q + v] & kSp) != 0;
-            anysp |= sp[v];
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+              for (int v = 0; v < VN; ++v) O.c[c].v[v] = fma_rn(m.c[c].v[v], K.c[c].v[v], O.c[c].v[v]);
+          } else {
+            update_cells<T, VN>(fxv, anyfx, xt, ry, rz, K, m, O, t, u);
           }
         }
-        if (!anysp) {
-          update_cells<T, VN>(fxv, anyfx, xtab + col, ry, rz, K, m, O, t, u);
-        } else {
-          Cells<T, VN> w;
-          if (anyfx) w.c[0] = get(p.W[0], 2128);
-          if (fy) w.c[1] = get(p.W[1], 2129);
-          if (fz) w.c[2] = get(p.W[2], 2119);
-          update_special_cells<T, VN>(sp, fxv, p.ax[0] + x0, p.ax[1] + j, cz.s, xtab + col, ry, rz, K, m, O, t, u, w);
-          if (anyfx) put(p.W[0] + q, w.c[0], 2131);
-          if (fy) put(p.W[1] + q, w.c[1], 2132);
-          if (fz) put(p.W[2] + q, w.c[2], 2133);
-        }
+      }
+      if (!plain) {
         // what was loaded goes back (values that a cell does not use unchanged)
         if (anyfx || tf) put(p.Ts[0] + q, t.c[0], 2121);
         if (fy || tf) put(p.Ts[1] + q, t.c[1], 2122);

@@ -162,6 +162,94 @@ __device__ __forceinline__ void update_cells(const bool (&fx)[VN], bool anyfx, c
   }
 }
 
+// Update of VN cells of a row without special cells, compiled for the CPMLs the
+// row can meet: WX its tile touches the x-CPML (fx[v]: cell v is in it, xt its
+// factors a, b, 1-σ, 1+σ, all 1 outside), FY and FZ the row or plane is in the y- or
+// z-CPML.  Straight-line: the cells of a row that differ only in fx[v] take both
+// forms and select, which costs a few operations; branching on fx cost both sides'
+// instructions and their registers.  t and u of cells that have none are read as
+// finite values and come back unchanged.
+template <bool WX, bool FY, bool FZ, typename T, int VN>
+__device__ __forceinline__ void update_row(const bool (&fx)[VN], const AxisCoef<T>* xt, const RedAxis<T>& ry,
+                                           const AxisCoef<T>& zt, const Cells<T, VN>& K, const Cells<T, VN>& m,
+                                           Cells<T, VN>& O, Cells<T, VN>& t, Cells<T, VN>& u) {
+  const T za = zt.s, zb = zt.om, zom = zt.ir, zop = zt.op;  // a, b, 1-σ, 1+σ
+#pragma unroll
+  for (int v = 0; v < VN; ++v) {
+    AxisCoef<T> x{T(1), T(1), T(1), T(1)};
+    bool f = false;
+    if constexpr (WX) {
+      x = xt[v];
+      f = fx[v];
+    }
+    const T xa = x.s, xb = x.om;
+    {  // component x: own axis x, next y, previous z
+      T d = K.c[0].v[v];
+      if constexpr (FY && FZ) {
+        const T un = fma_rn(ry.a, u.c[0].v[v], mul_rn(ry.b, d));
+        d = sub_rn(un, u.c[0].v[v]);
+        u.c[0].v[v] = un;
+      }
+      const T A = FZ ? za : ry.a, B = FZ ? zb : ry.b;
+      const T w = FY || FZ ? mul_rn(B, d) : d;
+      const T o = O.c[0].v[v], mm = m.c[0].v[v], tt = t.c[0].v[v];
+      T r = FY || FZ ? fma_rn(A, o, mul_rn(mm, w)) : fma_rn(mm, w, o);
+      if constexpr (WX) {
+        const T tn = FY || FZ ? fma_rn(A, tt, w) : add_rn(tt, w);
+        const T rt = fma_rn(mm, fma_rn(x.op, tn, -mul_rn(x.ir, tt)), o);
+        r = f ? rt : r;
+        t.c[0].v[v] = f ? tn : tt;
+      }
+      O.c[0].v[v] = r;
+    }
+    {  // component y: own axis y, next z, previous x
+      T d = K.c[1].v[v], A = za, B = zb;
+      if constexpr (WX && FZ) {
+        const T un = fma_rn(za, u.c[1].v[v], mul_rn(zb, d));
+        d = f ? sub_rn(un, u.c[1].v[v]) : d;
+        u.c[1].v[v] = f ? un : u.c[1].v[v];
+        A = f ? xa : za;
+        B = f ? xb : zb;
+      } else if constexpr (WX) {
+        A = xa;
+        B = xb;
+      }
+      constexpr bool damp = WX || FZ;
+      const T w = damp ? mul_rn(B, d) : d;
+      const T o = O.c[1].v[v], mm = m.c[1].v[v], tt = t.c[1].v[v];
+      if constexpr (FY) {
+        const T tn = damp ? fma_rn(A, tt, w) : add_rn(tt, w);
+        O.c[1].v[v] = fma_rn(mm, fma_rn(ry.op, tn, -mul_rn(ry.om, tt)), o);
+        t.c[1].v[v] = tn;
+      } else {
+        O.c[1].v[v] = damp ? fma_rn(A, o, mul_rn(mm, w)) : fma_rn(mm, w, o);
+      }
+    }
+    {  // component z: own axis z, next x, previous y
+      T d = K.c[2].v[v], A = xa, B = xb;
+      if constexpr (WX && FY) {
+        const T un = fma_rn(xa, u.c[2].v[v], mul_rn(xb, d));
+        d = f ? sub_rn(un, u.c[2].v[v]) : d;
+        u.c[2].v[v] = f ? un : u.c[2].v[v];
+      }
+      if constexpr (FY) {
+        A = ry.a;
+        B = ry.b;
+      }
+      constexpr bool damp = WX || FY;
+      const T w = damp ? mul_rn(B, d) : d;
+      const T o = O.c[2].v[v], mm = m.c[2].v[v], tt = t.c[2].v[v];
+      if constexpr (FZ) {
+        const T tn = damp ? fma_rn(A, tt, w) : add_rn(tt, w);
+        O.c[2].v[v] = fma_rn(mm, fma_rn(zop, tn, -mul_rn(zom, tt)), o);
+        t.c[2].v[v] = tn;
+      } else {
+        O.c[2].v[v] = damp ? fma_rn(A, o, mul_rn(mm, w)) : fma_rn(mm, w, o);
+      }
+    }
+  }
+}
+
 // Component of a special cell (source, χ3, pole): the complete state, T always,
 // U and W where its CPML stages have them.  has_w: own-axis CPML with σ ≠ 0, the
 // condition under which the sparse passes go through W (not to be read off the

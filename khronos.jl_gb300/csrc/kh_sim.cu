@@ -1972,7 +1972,7 @@ class Sim : public SimBase {
   int choose_zplanes() const {
     if (const char* zv = std::getenv("KHRONOS_GB300_ZPLANES")) {
       const int z = std::atoi(zv);
-      if (z >= 1) return std::min(z, n_[2]);
+      if (z >= 1) return std::min({z, n_[2], kh::kLeanZ});
     }
     // 10 planes: a measured optimum on 128- and 256-plane grids (one plane of
     // curl-source halo re-read per CTA against enough CTAs to balance the
