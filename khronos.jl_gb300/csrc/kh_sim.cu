@@ -1974,16 +1974,31 @@ class Sim : public SimBase {
       const int z = std::atoi(zv);
       if (z >= 1) return std::min({z, n_[2], kh::kLeanZ});
     }
-    // 10 planes: a measured optimum on 128- and 256-plane grids (one plane of
-    // curl-source halo re-read per CTA against enough CTAs to balance the
-    // SMs); shallower when the launch would not fill two rounds of resident CTAs.
-    int z = 10;
-    if (use_tma_ && tma_slots_ > 0) {
-      const long long xy = (long long)((n_[0] + kh::kLeanX - 1) / kh::kLeanX) * ((n_[1] + kh::kLeanY - 1) / kh::kLeanY);
-      const long long fill = xy * n_[2] / (2LL * tma_slots_);
-      z = int(std::max(2LL, std::min<long long>(z, fill)));
+    if (!use_tma_ || tma_slots_ <= 0) return std::min(10, n_[2]);
+    const long long xy =
+        (long long)((n_[0] + kh::kLeanX - 1) / kh::kLeanX) * ((n_[1] + kh::kLeanY - 1) / kh::kLeanY);
+    // FP64 is bound by arithmetic: the shallowest chunks balance best (240×144×96, 32
+    // steps: 12.26 / 12.40 / 12.50 / 12.52 / 13.0 ms at 2 / 3 / 4 / 5 / 10 planes).
+    if (sizeof(T) == 8) return std::min(2, n_[2]);
+    // A plane costs a CTA about 1.4 µs whatever else runs, its start about three
+    // planes; more rounds of CTAs cost less than their number (the SMs overlap them).
+    // The optimum of that grows with the square root of the rounds at one plane per
+    // CTA (320×192×128, 96 steps: 15.66 / 15.35 / 15.04 / 15.04 / 15.12 / 15.36 ms at 3 /
+    // 4 / 5 / 6 / 7 / 10 planes; 200×200×64: 23.97 / 23.58 / 22.96 / 23.07 / 23.40 at 3 - 7).
+    const double rounds = double(xy) * n_[2] / double(tma_slots_);
+    auto ctas = [&](int z) { return xy * ((n_[2] + z - 1) / z); };
+    const int best = int(std::max(2.0, std::min(7.0, std::floor(1.25 * std::sqrt(rounds) + 0.5))));
+    const double many = (best + 3) * (1.15 + 0.3 * double(ctas(best)) / double(tma_slots_));
+    // … unless all CTAs (but a few of the last, shorter ones) are resident at once at
+    // a depth that costs clearly less (96³, 64 steps: 3.87 ms at 5 planes, 4.05 at 2;
+    // 181×97×75, where it does not: 6.09 ms at 3 planes, 6.72 at 7).
+    for (int z = 1; z <= 10; ++z) {
+      const double r = double(ctas(z)) / double(tma_slots_);
+      if (r > 1.06) continue;
+      if ((z + 3) * (r > 1.0 ? 1.1 : 1.0) < 0.925 * many) return std::min(z, n_[2]);
+      break;
     }
-    return std::min(z, n_[2]);
+    return std::min(best, n_[2]);
   }
 
   // Whole-step launches on grids without CPML where nothing comes between the
