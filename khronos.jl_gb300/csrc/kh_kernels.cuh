@@ -334,14 +334,18 @@ int prepare_lean_kernels();
 template <typename T>
 int lean_resident_ctas();
 
-// History recording: copy one component over a cell box (x fastest) into a
-// contiguous slot of a history buffer.
+// History recording: the components of up to kMaxRecords monitors over their cell
+// boxes (x fastest) into a contiguous slot of each one's history buffer, in one launch.
+constexpr int kMaxRecords = 12;
 template <typename T>
 struct RecordParams {
-  const T* field;
   long long pitch, plane, origin, total;
-  int start[3], dims[3];
-  T* dst;
+  int n;
+  struct Rec {
+    const T* field;
+    int start[3], dims[3];
+    T* dst;
+  } rec[kMaxRecords];
 };
 
 template <typename T>

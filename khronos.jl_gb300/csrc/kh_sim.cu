@@ -1785,22 +1785,30 @@ class Sim : public SimBase {
   // History monitors of one half: the component values after that half-step
   // of step `ts` go to slot ts (steps past the capacity are not recorded).
   void record_histories(bool h_half, int64_t ts, cudaStream_t stream) {
-    for (auto& h : hists_) {
-      if ((h.comp >= 3) != h_half || ts >= h.cap) continue;
-      kh::RecordParams<T> p;
-      p.field = h.comp < 3 ? cur_E(h.comp) : cur_H(h.comp - 3);
-      p.pitch = pitch_;
-      p.plane = plane_;
-      p.origin = origin_;
-      p.total = total_;
-      for (int a = 0; a < 3; ++a) {
-        p.start[a] = h.start[a];
-        p.dims[a] = h.dims[a];
-      }
-      p.dst = h.buf + ts * h.ncell;
+    kh::RecordParams<T> p;
+    p.pitch = pitch_;
+    p.plane = plane_;
+    p.origin = origin_;
+    p.total = total_;
+    p.n = 0;
+    auto flush = [&]() {
+      if (p.n == 0) return;
       kh::launch_record<T>(p, stream);
       ++launches;
+      p.n = 0;
+    };
+    for (auto& h : hists_) {
+      if ((h.comp >= 3) != h_half || ts >= h.cap) continue;
+      auto& r = p.rec[p.n++];
+      r.field = h.comp < 3 ? cur_E(h.comp) : cur_H(h.comp - 3);
+      for (int a = 0; a < 3; ++a) {
+        r.start[a] = h.start[a];
+        r.dims[a] = h.dims[a];
+      }
+      r.dst = h.buf + ts * h.ncell;
+      if (p.n == kh::kMaxRecords) flush();
     }
+    flush();
   }
 
   // kh_sim_set_geometry: rasterise (and smooth) each E component's ε⁻¹ on the
