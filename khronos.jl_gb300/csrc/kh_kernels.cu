@@ -338,8 +338,15 @@ __device__ __forceinline__ void source_fix_one(const SourceFixParams<T>& p, long
   net += S;
   if (p.W[c]) {
     const long long rel = q - p.origin;
-    const long long k = rel / p.plane, rem = rel % p.plane;
-    const int idx = c == 0 ? int(rem % p.pitch) : (c == 1 ? int(rem / p.pitch) : int(k));
+    int idx;
+    if (p.total <= 0xffffffffll) {  // 32-bit division wherever the offsets fit
+      const unsigned r = unsigned(rel), plane = unsigned(p.plane), pitch = unsigned(p.pitch);
+      const unsigned k = r / plane, rem = r - k * plane, j = rem / pitch;
+      idx = int(c == 0 ? rem - j * pitch : (c == 1 ? j : k));
+    } else {
+      const long long k = rel / p.plane, rem = rel % p.plane;
+      idx = c == 0 ? int(rem % p.pitch) : (c == 1 ? int(rem / p.pitch) : int(k));
+    }
     if ((idx < p.pml_lo[c] || idx >= p.n[c] - p.pml_hi[c]) && KH_IN(idx, p.n[c], 3031)) {
       const AxisCoef<T> ao = p.ax[c][idx];
       if (ao.s != T(0)) {
@@ -614,13 +621,22 @@ __global__ void wrap_kernel(const WrapParams<T> p) {
   T* f = p.O[c];
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < face;
        e += (long long)gridDim.x * blockDim.x) {
-    const long long u = e % p.n[t1], v = e / p.n[t1];
+    long long u, v;
+    if (face <= 0xffffffffll) {  // 32-bit division wherever the face fits
+      const unsigned w = unsigned(e) / unsigned(p.n[t1]);
+      v = w;
+      u = unsigned(e) - w * unsigned(p.n[t1]);
+    } else {
+      u = e % p.n[t1];
+      v = e / p.n[t1];
+    }
     const long long base = p.origin + u * st[t1] + v * st[t2];
     const long long lo = base, hi = base + (long long)(p.n[a] - 1) * st[a];
     const long long ghost_lo = base - st[a], ghost_hi = base + (long long)p.n[a] * st[a];
     if (!(KH_IN(ghost_lo, p.total, 3028) && KH_IN(ghost_hi, p.total, 3029))) continue;
-    if (!(p.chi3 && p.chi3[hi] != T(0))) f[ghost_lo] = f[hi];
-    if (!(p.chi3 && p.chi3[lo] != T(0))) f[ghost_hi] = f[lo];
+    const T fh = f[hi], fl = f[lo];  // both on their way before the first store
+    if (!(p.chi3 && p.chi3[hi] != T(0))) f[ghost_lo] = fh;
+    if (!(p.chi3 && p.chi3[lo] != T(0))) f[ghost_hi] = fl;
   }
 }
 
