@@ -541,6 +541,16 @@ struct DispListArgs {
 };
 void launch_disp_list(const DispListArgs& a, void* stream);
 
+// Zero up to kMaxZero arrays (256-byte aligned, any length) in one launch.
+constexpr int kMaxZero = 64;
+struct ZeroArgs {
+  int n;
+  void* ptr[kMaxZero];
+  unsigned long long bytes[kMaxZero];
+  unsigned long long first[kMaxZero + 1];  // set by launch_zero: prefix sums of the arrays' 16 KB pieces
+};
+void launch_zero(ZeroArgs a, void* stream);
+
 // DFT accumulators (with Kahan compensation C, or nullptr) → interleaved
 // (re, im) doubles, value = F − C.
 template <typename T>

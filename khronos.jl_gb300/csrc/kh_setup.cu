@@ -142,6 +142,20 @@ __global__ void __launch_bounds__(kCompactThreads) compact_segments_kernel(const
   if (threadIdx.x == kCompactThreads - 1) *a.count = part[threadIdx.x];
 }
 
+// Pieces of 16 KB, one per block and turn; the array of a piece by its prefix sums.
+constexpr unsigned long long kZeroPiece = 16384;
+__global__ void __launch_bounds__(256) zero_kernel(const __grid_constant__ ZeroArgs a) {
+  for (unsigned long long u = blockIdx.x; u < a.first[a.n]; u += gridDim.x) {
+    int m = 0;
+    while (u >= a.first[m + 1]) ++m;
+    const unsigned long long b0 = (u - a.first[m]) * kZeroPiece;
+    const unsigned long long len = min(kZeroPiece, a.bytes[m] - b0);
+    char* p = static_cast<char*>(a.ptr[m]) + b0;
+    for (unsigned i = threadIdx.x; i < len / 16; i += 256) reinterpret_cast<uint4*>(p)[i] = make_uint4(0, 0, 0, 0);
+    if (threadIdx.x < len % 16) p[len / 16 * 16 + threadIdx.x] = 0;
+  }
+}
+
 template <typename T>
 __global__ void dft_read_kernel(const Cplx<T>* __restrict__ F, const Cplx<T>* __restrict__ C, double* out,
                                 long long n) {
@@ -195,6 +209,14 @@ void launch_disp_list(const DispListArgs& a, void* stream) {
   const int warps = 8;
   disp_flags_kernel<<<unsigned((nseg + warps - 1) / warps), 32 * warps, 0, static_cast<cudaStream_t>(stream)>>>(a);
   compact_segments_kernel<<<1, kCompactThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
+}
+
+void launch_zero(ZeroArgs a, void* stream) {
+  a.first[0] = 0;
+  for (int m = 0; m < a.n; ++m) a.first[m + 1] = a.first[m] + (a.bytes[m] + kZeroPiece - 1) / kZeroPiece;
+  if (a.n <= 0 || a.first[a.n] == 0) return;
+  const unsigned blocks = unsigned(std::min<unsigned long long>(a.first[a.n], 152ull * 16));
+  zero_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
 }
 
 template <typename T>
