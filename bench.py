@@ -359,7 +359,7 @@ def run_ours(args, world, rank, local_rank):
         return 0
     peak, peak_kind = measured_peaks()
     simt = os.environ.get("KHRONOS_GB300_KERNEL") == "simt"
-    e_kernel = "half_step_kernel<float,E>" if simt else "half_step_tma_kernel<float,E>"
+    e_kernel = "half_step_kernel<float,E>" if simt else "half_step_lean_kernel<float,E>"
     e_launch_ms = e_ms / rsteps
     achieved = e_bytes / (e_launch_ms / 1e3) / 1e9
     line = {

@@ -12,7 +12,7 @@
 // CPML: 48 µs a half-step for 262 MB, 5.5 TB/s); tiles in the CPML by the latency
 // of a plane (their auxiliaries' loads, then update, store and barrier) and its
 // instructions.  Against the complete cascade (T, U, W stored for every CPML cell)
-// a 320×192×128 step moves 771 instead of 970 MB, in 41 + 49 M instead of 64 + 66 M
+// a 320×192×128 step moves 757 instead of 978 MB, in 42 + 50 M instead of 64 + 66 M
 // warp instructions.
 //
 // Every mbarrier wait is bounded: after kSleepWaitLimit tries the thread records

@@ -1,4 +1,6 @@
-// TMA-staged fused half-step kernel for sm_103a.
+// General TMA-staged half-step kernel for sm_103a, on the complete CPML state: the
+// FULL variants (sources, χ3, poles, conductivity in-kernel) and the CPU-path
+// semantics.  The CUDA-path stages without these run in kh_lean.cu.
 //
 // Same arithmetic as the register-pipelined kernel (general_cell / pml_cell
 // of kh_cell.cuh), with the plane data moved by the Tensor Memory
