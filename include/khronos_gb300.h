@@ -412,7 +412,9 @@ kh_status kh_debug_bounds(int64_t* count, int64_t* index, int32_t* site);
 
 /* Device memory: what kh_sim_prepare will allocate (estimate, available
  * before prepare; estimate_memory, src/Memory.jl:120-251) and what it has
- * allocated (0 before prepare). */
+ * allocated (0 before prepare).  FP32 grids without CPML may add a second set of
+ * E and H on top of the estimate, only while that is below 1/16 of the free
+ * device memory and never for requests of a server. */
 kh_status kh_sim_memory_bytes(const kh_sim* sim, int64_t* estimate, int64_t* allocated);
 
 /* State control. */

@@ -332,7 +332,7 @@ void launch_half_step(bool h_half, const HalfStepParams<T>& p, void* stream) {
 // Component c of source cell q: O = m⁻¹·(T + S), or through the W stage
 // when the cell lies in the CPML of c's own axis (SourceFixParams).
 template <typename T>
-__device__ __forceinline__ void source_fix_one(const SourceFixParams<T>& p, long long q, int c, T S) {
+__device__ __forceinline__ T source_fix_cell(const SourceFixParams<T>& p, long long q, int c, T S) {
   const T m = p.m_inv[c] ? p.m_inv[c][q] : p.m_scalar;
   T net = p.Ts[c][q];
   net += S;
@@ -353,12 +353,35 @@ __device__ __forceinline__ void source_fix_one(const SourceFixParams<T>& p, long
         const T wl = p.W[c][q];
         const T wn = m * net;
         p.W[c][q] = wn;
-        p.O[c][q] = p.O[c][q] + ao.op * (wn - wl);
-        return;
+        const T o = p.O[c][q] + ao.op * (wn - wl);
+        p.O[c][q] = o;
+        return o;
       }
     }
   }
-  p.O[c][q] = m * net;
+  const T o = m * net;
+  p.O[c][q] = o;
+  return o;
+}
+
+template <typename T>
+__device__ __forceinline__ void source_fix_one(const SourceFixParams<T>& p, long long q, int c, T S) {
+  const T o = source_fix_cell(p, q, c, S);
+  if (!p.wrap) return;
+  // the ghost copies that the half-step made of a face cell
+  const long long rel = q - p.origin;
+  const int k = int(rel / p.plane);
+  const long long rem = rel - (long long)k * p.plane;
+  const int j = int(rem / p.pitch);
+  const int at[3] = {int(rem - (long long)j * p.pitch), j, k};
+  const long long st[3] = {1, p.pitch, p.plane};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    if (!((p.wrap >> a) & 1u)) continue;
+    const long long d = (long long)p.n[a] * st[a];
+    if (at[a] == 0 && KH_IN(q + d, p.total, 3032)) p.O[c][q + d] = o;
+    if (at[a] == p.n[a] - 1 && KH_IN(q - d, p.total, 3033)) p.O[c][q - d] = o;
+  }
 }
 
 template <typename T>
@@ -606,7 +629,8 @@ void launch_disp_fix(const DispFixParams<T>& p, void* stream) {
 }
 
 // ---------------------------------------------------------------------------
-// Periodic wrap.  One block row per periodic axis and component:
+// Periodic wrap after a half-step of the general or the register-pipelined kernel
+// (the reduced-state one writes its ghost layers itself).  One block row per periodic axis and component:
 // blockIdx.y = 3·(index of the axis in p.axes) + component; threads stride
 // over the face's (n_t1 × n_t2) cells, t1 the lower of the face's two axes;
 // each copies both directions of one cell.

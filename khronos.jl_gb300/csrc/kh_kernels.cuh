@@ -188,6 +188,9 @@ struct HalfStepParams {
   // its pre-correction E into the ghost layer the wrap fills (the reference
   // exchanges E before the Kerr correction); the wrap kernel skips those cells.
   uint32_t periodic;
+  // the same mask for the reduced-state kernel, which writes the ghost layers of
+  // its half itself
+  uint32_t wrap;
 
   int* err;  // set to KH_ERR_TIMEOUT by a kernel whose bounded wait gave up
   // Failure-detection test hook (0 in normal runs): nonzero launches the FP32
@@ -395,6 +398,7 @@ struct SourceFixParams {
   const AxisCoef<T>* ax[3];
   int n[3], pml_lo[3], pml_hi[3];
   long long pitch, plane, origin;
+  uint32_t wrap;  // periodic axes whose ghost layers the half-step wrote: repeated for source cells
 };
 
 // Dispersive and Kerr cells of a LEAN E half-step (the launch kept their D

@@ -50,7 +50,7 @@ struct LeanGeom {
 
 constexpr int kLeanThreads = kLeanY * kLeanX / kLeanVN;
 
-template <typename T, bool H, bool PV, bool STALL = false>
+template <typename T, bool H, bool PV, bool STALL = false, bool PER = false>
 __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
     half_step_lean_kernel(const __grid_constant__ HalfStepParams<T> p, const __grid_constant__ TmaMaps maps) {
   using G = LeanGeom<T, PV>;
@@ -322,6 +322,36 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
         put(o1, O.c[1], 2127);
         put(o2, O.c[2], 2127);
       }
+      if constexpr (PER) {
+        // periodic axes: the face cells also into the ghost layer across (layer 0
+        // into n, layer n - 1 into -1, over the cells of the other two axes), instead
+        // of a wrap launch after each half (256×256×128, x and y, 64 steps: 10.96 to
+        // 10.04 ms; 64³ 21.5 to 17.5 µs a step)
+        if ((p.wrap & 1u) && (x0 == 0 || x0 + VN >= p.nx)) {
+          T* const o[3] = {o0, o1, o2};
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int v = 0; v < VN; ++v) {
+              if (x0 + v == 0 && KH_IN(q + p.nx, p.total, 2140)) o[c][p.nx] = O.c[c].v[v];
+              if (x0 + v == p.nx - 1 && KH_IN(q + v - p.nx, p.total, 2141)) o[c][v - p.nx] = O.c[c].v[v];
+            }
+        }
+        auto across = [&](bool lo, bool hi, long long d) {
+          if (lo && KH_IN(q + d + VN - 1, p.total, 2142)) {
+            put(o0 + d, O.c[0], 2143);
+            put(o1 + d, O.c[1], 2143);
+            put(o2 + d, O.c[2], 2143);
+          }
+          if (hi && KH_IN(q - d, p.total, 2144)) {
+            put(o0 - d, O.c[0], 2145);
+            put(o1 - d, O.c[1], 2145);
+            put(o2 - d, O.c[2], 2145);
+          }
+        };
+        if (p.wrap & 2u) across(j == 0, j == p.ny - 1, (long long)p.ny * p.pitch);
+        if (p.wrap & 4u) across(k == 0, k == p.nz - 1, (long long)p.nz * p.plane);
+      }
     }
     q += step;
     o0 += step;
@@ -390,7 +420,8 @@ static void launch_lean_variant(const HalfStepParams<T>& p, const TmaMaps& maps,
       return;
     }
   }
-  half_step_lean_kernel<T, H, PV><<<grid, block, LeanGeom<T, PV>::SMEM, st>>>(p, maps);
+  if (p.wrap) half_step_lean_kernel<T, H, PV, false, true><<<grid, block, LeanGeom<T, PV>::SMEM, st>>>(p, maps);
+  else half_step_lean_kernel<T, H, PV><<<grid, block, LeanGeom<T, PV>::SMEM, st>>>(p, maps);
 }
 
 template <typename T>
@@ -406,9 +437,9 @@ void launch_half_step_lean(bool h_half, const HalfStepParams<T>& p, const TmaMap
   }
 }
 
-template <typename T, bool H, bool PV, bool STALL = false>
+template <typename T, bool H, bool PV, bool STALL = false, bool PER = false>
 static int set_lean_attr() {
-  return int(cudaFuncSetAttribute(half_step_lean_kernel<T, H, PV, STALL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return int(cudaFuncSetAttribute(half_step_lean_kernel<T, H, PV, STALL, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   int(LeanGeom<T, PV>::SMEM)));
 }
 
@@ -419,6 +450,10 @@ int prepare_lean_kernels() {
   e |= set_lean_attr<T, true, false>();
   e |= set_lean_attr<T, false, true>();
   e |= set_lean_attr<T, false, false>();
+  e |= set_lean_attr<T, true, true, false, true>();
+  e |= set_lean_attr<T, true, false, false, true>();
+  e |= set_lean_attr<T, false, true, false, true>();
+  e |= set_lean_attr<T, false, false, false, true>();
   if constexpr (sizeof(T) == 4) {
     e |= set_lean_attr<T, true, true, true>();
     e |= set_lean_attr<T, true, false, true>();

@@ -1669,7 +1669,7 @@ class Sim : public SimBase {
         kh::launch_source_fix<T>(fh, st);
         ++launches;
       }
-      if (d_.periodic) {
+      if (d_.periodic && (ph.full || !reduced_[1])) {
         kh::launch_wrap<T>(wh, st);
         ++launches;
       }
@@ -1686,7 +1686,7 @@ class Sim : public SimBase {
       else kh::launch_half_step<T>(false, pe, st);
       ++launches;
       after_e(P, st);
-      if (d_.periodic) {
+      if (d_.periodic && (pe.full || !reduced_[0])) {
         kh::launch_wrap<T>(we, st);
         ++launches;
       }
@@ -2161,6 +2161,7 @@ class Sim : public SimBase {
     }
     f.m_scalar = h ? T(d_.mu_inv) : T(d_.eps_inv);
     f.h_half = h ? 1 : 0;
+    f.wrap = reduced_[h ? 1 : 0] ? uint32_t(d_.periodic) : 0u;
     if (d_.semantics == KH_SEM_CPML)
       for (int c = 0; c < 3; ++c) f.W[c] = h ? WB_[c] : WD_[c];
     for (int a = 0; a < 3; ++a) {
@@ -2272,6 +2273,7 @@ class Sim : public SimBase {
     p.err = err_dev_;
     p.stall_tx = stall_tx_;
     p.periodic = h ? 0u : uint32_t(d_.periodic);
+    p.wrap = reduced_[h ? 1 : 0] ? uint32_t(d_.periodic) : 0u;
     p.slot_off = slot_off_;
     p.ent_src = ent_src_;
     p.ent_comp = ent_comp_;
