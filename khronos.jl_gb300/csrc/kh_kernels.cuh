@@ -331,6 +331,18 @@ template <typename T>
 void launch_half_step_lean(bool h_half, const HalfStepParams<T>& p, const TmaMaps& maps, void* stream);
 template <typename T>
 void launch_expand_state(bool h_half, const HalfStepParams<T>& p, void* stream);
+// A complete state against what the reduced one takes for granted in CPML cells
+// without special state: broken, W = m·T (own axis) or O = m·T (outside it) does not
+// hold to rounding; off_u against top_t, the largest |U - T| where only the next axis
+// damps (U is then not kept); off_o against top_o, the largest |O - m·T| where the
+// own axis has σ = 0.  All zero before the launch.
+template <typename T>
+struct StateCheck {
+  T top_t, off_u, top_o, off_o;
+  int broken;
+};
+template <typename T>
+void launch_check_state(bool h_half, const HalfStepParams<T>& p, StateCheck<T>* out, void* stream);
 template <typename T>
 int prepare_lean_kernels();
 // CTAs of the reduced-state kernel resident on one SM (after prepare).

@@ -21,6 +21,9 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
+
 #include "../../include/khronos_gb300.h"
 #include "kh_async.cuh"
 #include "kh_lean.cuh"
@@ -410,6 +413,68 @@ void launch_expand_state(bool h_half, const HalfStepParams<T>& p, void* stream) 
   else expand_state_kernel<T, false><<<grid, 128, 0, st>>>(p);
 }
 
+// What the reduced state takes for granted, checked on the complete T, U and W of a
+// state from elsewhere (StateCheck, kh_kernels.cuh).
+template <typename T, bool H>
+__global__ void check_state_kernel(const HalfStepParams<T> p, StateCheck<T>* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= p.nx) return;
+  const T eps = sizeof(T) == 4 ? T(1.1920929e-7) : T(2.220446049250313e-16);
+  const T tiny = sizeof(T) == 4 ? T(1.17549435e-38) : T(2.2250738585072014e-308);
+  bool broken = false;
+  T top_t = T(0), off_u = T(0), top_o = T(0), off_o = T(0);
+  // the largest so far; NaN counts as infinite
+  auto most = [](T& m, T x) {
+    if (!(x <= m)) m = x == x ? x : T(INFINITY);
+  };
+  for (int k = blockIdx.z; k < p.nz; k += gridDim.z)
+    for (int j = blockIdx.y; j < p.ny; j += gridDim.y) {
+      const bool f[3] = {i < p.pml_lo[0] || i >= p.nx - p.pml_hi[0], j < p.pml_lo[1] || j >= p.ny - p.pml_hi[1],
+                         k < p.pml_lo[2] || k >= p.nz - p.pml_hi[2]};
+      if (!(f[0] || f[1] || f[2])) continue;
+      const long long q = p.origin + (long long)k * p.plane + (long long)j * p.pitch + i;
+      if (!KH_IN(q, p.total, 2150)) continue;
+      if (p.cell_class && (p.cell_class[q] & (H ? kSpecialH : kSpecialE))) continue;  // keeps the complete state
+      const int idx[3] = {i, j, k};
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const int n = (c + 1) % 3, v = (c + 2) % 3;
+        const T t = p.Ts[c][q], o = p.O[c][q];
+        const T mt = mul_rn(p.m_inv[c] ? p.m_inv[c][q] : p.m_scalar, t);
+        const T near = T(8) * (eps * fabs(mt) + tiny);
+        if (f[c] && p.ax[c][idx[c]].s != T(0)) {
+          broken |= !(fabs(p.W[c][q] - mt) <= near);
+        } else if (!f[c]) {
+          broken |= !(fabs(o - mt) <= near);
+        } else {  // σ = 0: O goes on by differences, apart from m·T by their rounding
+          most(top_o, fabs(o));
+          most(off_o, fabs(o - mt));
+        }
+        if (f[n] && !f[v] && p.ax[n][idx[n]].s != T(0)) {
+          most(top_t, fabs(t));
+          most(off_u, fabs(p.U[c][q] - t));
+        }
+      }
+    }
+  if (broken) atomicOr(&out->broken, 1);
+  auto raise = [](T* a, T x) {  // non-negative values order like their bits
+    if constexpr (sizeof(T) == 4) atomicMax(reinterpret_cast<int*>(a), __float_as_int(x));
+    else atomicMax(reinterpret_cast<long long*>(a), __double_as_longlong(x));
+  };
+  if (top_t > T(0)) raise(&out->top_t, top_t);
+  if (off_u > T(0)) raise(&out->off_u, off_u);
+  if (top_o > T(0)) raise(&out->top_o, top_o);
+  if (off_o > T(0)) raise(&out->off_o, off_o);
+}
+
+template <typename T>
+void launch_check_state(bool h_half, const HalfStepParams<T>& p, StateCheck<T>* out, void* stream) {
+  const dim3 grid((p.nx + 127) / 128, std::min(p.ny, 65535), std::min(p.nz, 256));
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (h_half) check_state_kernel<T, true><<<grid, 128, 0, st>>>(p, out);
+  else check_state_kernel<T, false><<<grid, 128, 0, st>>>(p, out);
+}
+
 template <typename T, bool H, bool PV>
 static void launch_lean_variant(const HalfStepParams<T>& p, const TmaMaps& maps, cudaStream_t st) {
   const dim3 block(kLeanThreads, 1, 1);
@@ -476,6 +541,8 @@ template void launch_half_step_lean<float>(bool, const HalfStepParams<float>&, c
 template void launch_half_step_lean<double>(bool, const HalfStepParams<double>&, const TmaMaps&, void*);
 template void launch_expand_state<float>(bool, const HalfStepParams<float>&, void*);
 template void launch_expand_state<double>(bool, const HalfStepParams<double>&, void*);
+template void launch_check_state<float>(bool, const HalfStepParams<float>&, StateCheck<float>*, void*);
+template void launch_check_state<double>(bool, const HalfStepParams<double>&, StateCheck<double>*, void*);
 template int prepare_lean_kernels<float>();
 template int prepare_lean_kernels<double>();
 template int lean_resident_ctas<float>();

@@ -1197,8 +1197,7 @@ class Sim : public SimBase {
     if (kh_status es = wait_idle(); es != KH_OK) return es;
     if (kh_status es = expand_state(); es != KH_OK) return es;
     char* p = static_cast<char*>(dst);
-    // bit 0: sources active, bit 1: the run goes on from the complete state
-    int64_t hdr[2] = {timestep_, (sources_active_ ? 1 : 0) | (complete_state_ ? 2 : 0)};
+    int64_t hdr[2] = {timestep_, sources_active_ ? 1 : 0};
     std::memcpy(p, hdr, 16);
     p += 16;
     for (auto& s : state_) {
@@ -1221,8 +1220,7 @@ class Sim : public SimBase {
     }
     timestep_ = hdr[0];
     sources_active_ = (hdr[1] & 1) != 0;
-    complete_state_ = (hdr[1] & 2) != 0 && (reduced_[0] || reduced_[1]);
-    return KH_OK;
+    return check_imported();
   }
 
   // Compulsory-traffic model: the reference's 9 + 12 words per cell
@@ -2116,6 +2114,35 @@ class Sim : public SimBase {
   T* cur_E(int c) const { return cur_ ? E2_[c] : E_[c]; }
   T* cur_H(int c) const { return cur_ ? H2_[c] : H_[c]; }
 
+  // A state may come from a simulation with other materials or another absorber, or
+  // from this one before its materials changed: W, O and U are then not what the
+  // reduced state derives from T, and the run goes on from the complete state.
+  kh_status check_imported() {
+    complete_state_ = false;
+    if (!(reduced_[0] || reduced_[1]) || !(pml_axis_[0] || pml_axis_[1] || pml_axis_[2])) return KH_OK;
+    kh::StateCheck<T> c[2];
+    std::memset(c, 0, sizeof(c));
+    kh::StateCheck<T>* dev = nullptr;
+    KH_CUDA(kh_host::dev_alloc((void**)&dev, sizeof(c), cudaStreamLegacy));
+    cudaError_t e = cudaMemsetAsync(dev, 0, sizeof(c), cudaStreamLegacy);
+    for (int h = 0; h < 2 && e == cudaSuccess; ++h) {
+      if (!reduced_[h]) continue;
+      kh::launch_check_state<T>(h == 1, base_params(h == 1), dev + h, cudaStreamLegacy);
+      ++launches;
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(c, dev, sizeof(c), cudaMemcpyDeviceToHost);
+    kh_host::dev_free(dev, cudaStreamLegacy);
+    if (e != cudaSuccess) return fail(KH_ERR_CUDA, std::string("state check: ") + cudaGetErrorString(e));
+    // U and T (and O and m·T where σ = 0) part by the rounding of a run; a real
+    // difference is of their own size
+    const T drift = sizeof(T) == 4 ? T(1e-3) : T(1e-9);
+    for (int h = 0; h < 2; ++h)
+      if (reduced_[h] && (c[h].broken || !(c[h].off_u <= drift * c[h].top_t) || !(c[h].off_o <= drift * c[h].top_o)))
+        complete_state_ = true;
+    return KH_OK;
+  }
+
   // T, U and W of every CPML cell brought up to date from the reduced state.
   kh_status expand_state() {
     if (complete_state_ || !(pml_axis_[0] || pml_axis_[1] || pml_axis_[2])) return KH_OK;
@@ -2359,8 +2386,9 @@ class Sim : public SimBase {
   // [E half, H half]: the reduced-state kernel takes this half's launches.  T, U
   // and W that follow from the rest of the state are then not kept up to date.
   bool reduced_[2] = {false, false};
-  // A material of a CPML cell changed mid-run, so W = m·T no longer holds: the
-  // general kernel carries on from the complete state until reset().
+  // W, O or U of a CPML cell is not what the reduced state derives from T (a material
+  // changed mid-run, a state imported from elsewhere): the general kernel carries on
+  // from the complete state until reset() or the next import.
   bool complete_state_ = false;
   // Whole-step launches (kh_fused.cu): the second set of E and H, the tensor maps
   // from set 0 into 1 and back, and the set that holds the current fields (1 only
