@@ -1051,13 +1051,14 @@ class Sim : public SimBase {
       if (dm[a] <= 0 || st[a] < 0 || st[a] + dm[a] > n_[a]) return fail(KH_ERR_INVALID, "box outside the grid");
     if (kh_status es = wait_idle(); es != KH_OK) return es;
     // mid-run in a CPML cell of a half on the reduced state: W keeps the old
-    // material's value for one step, so the run goes on from the complete state
-    if (timestep_ > 0 && reduced_[kind == KH_MAT_MU_INV ? 1 : 0] && !complete_state_) {
+    // material's value for one step, which goes through the complete state
+    const int half = kind == KH_MAT_MU_INV ? 1 : 0;
+    if (timestep_ > 0 && reduced_[half] && complete_[half] == kDerived) {
       bool cpml = false;
       for (int a = 0; a < 3; ++a) cpml = cpml || st[a] < lo_[a] || st[a] + dm[a] > n_[a] - hi_[a];
       if (cpml) {
         if (kh_status es = expand_state(); es != KH_OK) return es;
-        complete_state_ = true;
+        complete_[half] = kOneStep;
       }
     }
     std::vector<T> plane(size_t(dm[0]) * dm[1]);
@@ -1182,7 +1183,7 @@ class Sim : public SimBase {
     KH_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     timestep_ = 0;
     sources_active_ = true;
-    complete_state_ = false;
+    complete_[0] = complete_[1] = kDerived;
     return KH_OK;
   }
 
@@ -1608,11 +1609,13 @@ class Sim : public SimBase {
     const bool msb = msigb_[0] || msigb_[1] || msigb_[2];
     const bool msd = msigd_[0] || msigd_[1] || msigd_[2];
     const bool ref_cpu = d_.semantics == KH_SEM_REFERENCE_CPU;
-    const bool full_h_base = msb || (ref_cpu && special_in_region_[1]) || complete_state_;
+    // … and on the complete state: every step, or the first one of the batch
+    auto complete = [&](int h, int s) { return complete_[h] == kStays || (complete_[h] == kOneStep && s == 0); };
+    const bool full_h_base = msb || (ref_cpu && special_in_region_[1]);
     // χ3 and pole cells: in the LEAN E launch plus the dispersive-cell pass
     // (disp_fix_), or in the FULL launch
     const bool dispersive = chi3_ != nullptr || !poles_d_.empty();
-    const bool full_e_base = msd || (dispersive && !disp_fix_) || (ref_cpu && special_in_region_[0]) || complete_state_;
+    const bool full_e_base = msd || (dispersive && !disp_fix_) || (ref_cpu && special_in_region_[0]);
     const kh::WrapParams<T> wh = wrap_params(true), we = wrap_params(false);
     kh::SourceFixParams<T> fh = fix_params(true), fe = fix_params(false);
     kh::DispFixParams<T> dfix = disp_params(pe);
@@ -1632,7 +1635,7 @@ class Sim : public SimBase {
         ++launches;
       }
     };
-    const bool whole = fused_ && !timing && !complete_state_;
+    const bool whole = fused_ && !timing;
     auto issue_all = [&](cudaStream_t st) {
     for (int s = 0; s < nb; ++s) {
       // two whole steps, into the second set and back
@@ -1656,7 +1659,7 @@ class Sim : public SimBase {
       ph.sources_active = P.sa ? 1 : 0;
       ph.f_now = dtab + P.fH;
       const bool src_h = P.sa && has_src_[1];
-      ph.full = (full_h_base || (src_h && !src_lean_ok_[1])) ? 1 : 0;
+      ph.full = (full_h_base || (src_h && !src_lean_ok_[1]) || complete(1, s)) ? 1 : 0;
       mark(s, 0);
       if (reduced_[1] && !ph.full) kh::launch_half_step_lean<T>(true, ph, lean_maps_h_, st);
       else if (use_tma_) kh::launch_half_step_tma<T>(true, ph, maps_h_, st);
@@ -1678,7 +1681,7 @@ class Sim : public SimBase {
       pe.sources_active = P.sa ? 1 : 0;
       pe.f_now = dtab + P.fE;
       const bool src_e = P.sa && has_src_[0];
-      pe.full = (full_e_base || (src_e && !src_lean_ok_[0])) ? 1 : 0;
+      pe.full = (full_e_base || (src_e && !src_lean_ok_[0]) || complete(0, s)) ? 1 : 0;
       if (reduced_[0] && !pe.full) kh::launch_half_step_lean<T>(false, pe, lean_maps_e_, st);
       else if (use_tma_) kh::launch_half_step_tma<T>(false, pe, maps_e_, st);
       else kh::launch_half_step<T>(false, pe, st);
@@ -1703,7 +1706,7 @@ class Sim : public SimBase {
       sig.reserve(size_t(nb) * 8 + 4);
       sig.push_back(nb);
       sig.push_back(b);
-      sig.push_back(complete_state_ ? 1 : 0);
+      sig.push_back(complete_[0] + 4 * complete_[1]);
       for (int q = 0; q < nb; ++q) {
         const StepPlan& P = plan[q];
         sig.push_back(P.sa ? 1 : 0);
@@ -1772,6 +1775,8 @@ class Sim : public SimBase {
     batch_recorded_ = true;
     last_stream_ = stream;
     timestep_ += nb;
+    for (int h = 0; h < 2; ++h)
+      if (complete_[h] == kOneStep) complete_[h] = kDerived;
     if (timing) {
       KH_CUDA(cudaEventSynchronize(batch_done_));
       for (int s = 0; s < nb; ++s) {
@@ -2116,9 +2121,10 @@ class Sim : public SimBase {
 
   // A state may come from a simulation with other materials or another absorber, or
   // from this one before its materials changed: W, O and U are then not what the
-  // reduced state derives from T, and the run goes on from the complete state.
+  // reduced state derives from T, and the run goes on from the complete state.  One
+  // step there makes W = m·T and O = m·T again; U - T stays as it is.
   kh_status check_imported() {
-    complete_state_ = false;
+    complete_[0] = complete_[1] = kDerived;
     if (!(reduced_[0] || reduced_[1]) || !(pml_axis_[0] || pml_axis_[1] || pml_axis_[2])) return KH_OK;
     kh::StateCheck<T> c[2];
     std::memset(c, 0, sizeof(c));
@@ -2137,17 +2143,19 @@ class Sim : public SimBase {
     // U and T (and O and m·T where σ = 0) part by the rounding of a run; a real
     // difference is of their own size
     const T drift = sizeof(T) == 4 ? T(1e-3) : T(1e-9);
-    for (int h = 0; h < 2; ++h)
-      if (reduced_[h] && (c[h].broken || !(c[h].off_u <= drift * c[h].top_t) || !(c[h].off_o <= drift * c[h].top_o)))
-        complete_state_ = true;
+    for (int h = 0; h < 2; ++h) {
+      if (!reduced_[h]) continue;
+      if (!(c[h].off_u <= drift * c[h].top_t)) complete_[h] = kStays;
+      else if (c[h].broken || !(c[h].off_o <= drift * c[h].top_o)) complete_[h] = kOneStep;
+    }
     return KH_OK;
   }
 
   // T, U and W of every CPML cell brought up to date from the reduced state.
   kh_status expand_state() {
-    if (complete_state_ || !(pml_axis_[0] || pml_axis_[1] || pml_axis_[2])) return KH_OK;
+    if (!(pml_axis_[0] || pml_axis_[1] || pml_axis_[2])) return KH_OK;
     for (int h = 0; h < 2; ++h) {
-      if (!reduced_[h]) continue;
+      if (!reduced_[h] || complete_[h] != kDerived) continue;
       kh::launch_expand_state<T>(h == 1, base_params(h == 1), cudaStreamLegacy);
       ++launches;
     }
@@ -2386,10 +2394,12 @@ class Sim : public SimBase {
   // [E half, H half]: the reduced-state kernel takes this half's launches.  T, U
   // and W that follow from the rest of the state are then not kept up to date.
   bool reduced_[2] = {false, false};
-  // W, O or U of a CPML cell is not what the reduced state derives from T (a material
-  // changed mid-run, a state imported from elsewhere): the general kernel carries on
-  // from the complete state until reset() or the next import.
-  bool complete_state_ = false;
+  // [E half, H half]: kDerived, unless W, O or U of a CPML cell is not what the reduced
+  // state derives from T: the general kernel then does one step from the complete state
+  // (a material changed mid-run), or all steps until reset() or the next import (U of an
+  // imported state is another absorber's).
+  enum { kDerived = 0, kOneStep = 1, kStays = 2 };
+  int complete_[2] = {kDerived, kDerived};
   // Whole-step launches (kh_fused.cu): the second set of E and H, the tensor maps
   // from set 0 into 1 and back, and the set that holds the current fields (1 only
   // between the two steps of a pair).
