@@ -42,7 +42,7 @@ def _stale(lib: Path = LIB) -> bool:
     if not lib.exists():
         return True
     t = lib.stat().st_mtime
-    deps = [CSRC / s for s in SOURCES] + [CSRC / h for h in ("kh_kernels.cuh", "kh_cell.cuh", "kh_async.cuh", "kh_lean.cuh", "kh_simbase.h")] + [ROOT / "include" / "khronos_gb300.h"]
+    deps = [CSRC / s for s in SOURCES] + [CSRC / h for h in ("kh_kernels.cuh", "kh_cell.cuh", "kh_async.cuh", "kh_lean.cuh", "kh_plan.h", "kh_simbase.h")] + [ROOT / "include" / "khronos_gb300.h"]
     return any(d.stat().st_mtime > t for d in deps)
 
 

@@ -324,6 +324,9 @@ void launch_half_step_tma(bool h_half, const HalfStepParams<T>& p, const TmaMaps
 // Kernel attribute set-up (dynamic shared memory size), once per device.
 template <typename T>
 int prepare_tma_kernels();
+// CTAs of the general kernel resident on one SM (after prepare).
+template <typename T>
+int tma_resident_ctas();
 
 // Reduced-state half-step (kh_lean.cu) for the CUDA-path CPML stages; its maps
 // have boxes of kLeanY rows.  expand: the complete T, U, W from its state.

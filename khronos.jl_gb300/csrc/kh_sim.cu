@@ -23,6 +23,7 @@
 
 #include "../../include/khronos_gb300.h"
 #include "kh_kernels.cuh"
+#include "kh_plan.h"
 #include "kh_simbase.h"
 
 #include <cudaTypedefs.h>
@@ -778,7 +779,7 @@ class Sim : public SimBase {
     const char* bv = std::getenv("KHRONOS_GB300_DFT_BATCH");
     dft_batch_ = !(bv && std::string(bv) == "0");
     if (use_tma_) KH_TRY(build_tma_maps());
-    zplanes_ = choose_zplanes();
+    choose_zplanes();
     if (const char* xv = std::getenv("KHRONOS_GB300_XPREFETCH")) xprefetch_ = std::min(2, std::max(0, std::atoi(xv)));
     if (const char* dv = std::getenv("KHRONOS_GB300_XPF_DIST")) xpf_dist_ = std::min(8, std::max(1, std::atoi(dv)));
     if (const char* sv = std::getenv("KHRONOS_GB300_TEST_STALL")) stall_tx_ = std::string(sv) == "1" ? 16u : 0u;
@@ -1661,6 +1662,7 @@ class Sim : public SimBase {
       const bool src_h = P.sa && has_src_[1];
       ph.full = (full_h_base || (src_h && !src_lean_ok_[1]) || complete(1, s)) ? 1 : 0;
       mark(s, 0);
+      ph.zplanes = reduced_[1] && !ph.full ? zplanes_ : general_zplanes_;
       if (reduced_[1] && !ph.full) kh::launch_half_step_lean<T>(true, ph, lean_maps_h_, st);
       else if (use_tma_) kh::launch_half_step_tma<T>(true, ph, maps_h_, st);
       else kh::launch_half_step<T>(true, ph, st);
@@ -1682,6 +1684,7 @@ class Sim : public SimBase {
       pe.f_now = dtab + P.fE;
       const bool src_e = P.sa && has_src_[0];
       pe.full = (full_e_base || (src_e && !src_lean_ok_[0]) || complete(0, s)) ? 1 : 0;
+      pe.zplanes = reduced_[0] && !pe.full ? zplanes_ : general_zplanes_;
       if (reduced_[0] && !pe.full) kh::launch_half_step_lean<T>(false, pe, lean_maps_e_, st);
       else if (use_tma_) kh::launch_half_step_tma<T>(false, pe, maps_e_, st);
       else kh::launch_half_step<T>(false, pe, st);
@@ -1958,7 +1961,8 @@ class Sim : public SimBase {
     int sms = 0;
     KH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     if (sizeof(T) == 4) fused_slots_ = sms * kh::fused_resident_ctas<float>();
-    tma_slots_ = sms * kh::lean_resident_ctas<T>();
+    lean_slots_ = sms * kh::lean_resident_ctas<T>();
+    tma_slots_ = sms * kh::tma_resident_ctas<T>();
     const int hx = 16 / int(sizeof(T));
     struct MapSet {
       kh::TmaMaps *h, *e;
@@ -1990,37 +1994,20 @@ class Sim : public SimBase {
     return KH_OK;
   }
 
-  // z planes per CTA of the TMA-staged kernel; KHRONOS_GB300_ZPLANES overrides.
-  int choose_zplanes() const {
+  // z planes per CTA of the reduced-state and of the general half-step kernel.
+  void choose_zplanes() {
+    zplanes_ = general_zplanes_ = std::min(10, n_[2]);
+    if (use_tma_) {
+      zplanes_ = kh::reduced_zplanes(n_[2], kh::plan_tiles(n_[0], n_[1], kh::kLeanX, kh::kLeanY), lean_slots_, sizeof(T) == 8);
+      general_zplanes_ = kh::general_zplanes(n_[2], kh::plan_tiles(n_[0], n_[1], kh::kTmaX, kh::kTmaY), tma_slots_);
+    }
     if (const char* zv = std::getenv("KHRONOS_GB300_ZPLANES")) {
       const int z = std::atoi(zv);
-      if (z >= 1) return std::min({z, n_[2], kh::kLeanZ});
+      if (z >= 1) {
+        zplanes_ = std::min({z, n_[2], kh::kLeanZ});
+        general_zplanes_ = std::min(z, n_[2]);
+      }
     }
-    if (!use_tma_ || tma_slots_ <= 0) return std::min(10, n_[2]);
-    const long long xy =
-        (long long)((n_[0] + kh::kLeanX - 1) / kh::kLeanX) * ((n_[1] + kh::kLeanY - 1) / kh::kLeanY);
-    // FP64 is bound by arithmetic: the shallowest chunks balance best (240×144×96, 32
-    // steps: 12.26 / 12.40 / 12.50 / 12.52 / 13.0 ms at 2 / 3 / 4 / 5 / 10 planes).
-    if (sizeof(T) == 8) return std::min(2, n_[2]);
-    // A plane costs a CTA about 1.4 µs whatever else runs, its start about three
-    // planes; more rounds of CTAs cost less than their number (the SMs overlap them).
-    // The optimum of that grows with the square root of the rounds at one plane per
-    // CTA (320×192×128, 96 steps: 15.66 / 15.35 / 15.04 / 15.04 / 15.12 / 15.36 ms at 3 /
-    // 4 / 5 / 6 / 7 / 10 planes; 200×200×64: 23.97 / 23.58 / 22.96 / 23.07 / 23.40 at 3 - 7).
-    const double rounds = double(xy) * n_[2] / double(tma_slots_);
-    auto ctas = [&](int z) { return xy * ((n_[2] + z - 1) / z); };
-    const int best = int(std::max(2.0, std::min(7.0, std::floor(1.25 * std::sqrt(rounds) + 0.5))));
-    const double many = (best + 3) * (1.15 + 0.3 * double(ctas(best)) / double(tma_slots_));
-    // … unless all CTAs (but a few of the last, shorter ones) are resident at once at
-    // a depth that costs clearly less (96³, 64 steps: 3.87 ms at 5 planes, 4.05 at 2;
-    // 181×97×75, where it does not: 6.09 ms at 3 planes, 6.72 at 7).
-    for (int z = 1; z <= 10; ++z) {
-      const double r = double(ctas(z)) / double(tma_slots_);
-      if (r > 1.06) continue;
-      if ((z + 3) * (r > 1.0 ? 1.1 : 1.0) < 0.925 * many) return std::min(z, n_[2]);
-      break;
-    }
-    return std::min(best, n_[2]);
   }
 
   // Whole-step launches on grids without CPML where nothing comes between the
@@ -2275,7 +2262,6 @@ class Sim : public SimBase {
     p.origin = origin_;
     p.total = total_;
     p.nxb = nxb_;
-    p.zplanes = zplanes_;
     p.xprefetch = xprefetch_;
     p.xpf_dist = xpf_dist_;
     p.dt = dt_;
@@ -2384,11 +2370,11 @@ class Sim : public SimBase {
   bool disp_fix_ = false;      // χ3 / pole cells by the dispersive-cell pass after a LEAN E launch
   uint32_t* disp_list_ = nullptr;  // its row-segment list (DispFixParams::list)
   int n_disp_list_ = 0;
-  int zplanes_ = 10;
+  int zplanes_ = 10, general_zplanes_ = 10;  // of kh_lean.cu, of kh_tma.cu
   int xprefetch_ = 2;        // x-CPML state prefetch mode (HalfStepParams::xprefetch)
   int xpf_dist_ = 3;
   int fused_slots_ = 1;  // SMs × resident whole-step CTAs per SM
-  int tma_slots_ = 0;  // SMs × resident TMA-kernel CTAs per SM
+  int lean_slots_ = 1, tma_slots_ = 1;  // … reduced-state, general-kernel CTAs per SM
   kh::TmaMaps maps_h_, maps_e_;            // kTmaY rows (general kernel)
   kh::TmaMaps lean_maps_h_, lean_maps_e_;  // kLeanY rows (reduced-state kernel)
   // [E half, H half]: the reduced-state kernel takes this half's launches.  T, U

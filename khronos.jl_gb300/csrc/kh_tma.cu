@@ -470,11 +470,22 @@ int prepare_tma_kernels() {
   return e;
 }
 
+template <typename T>
+int tma_resident_ctas() {
+  int n = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, half_step_tma_kernel<T, true, false, false>, 32 * kTmaY,
+                                                    TmaGeom<T>::SMEM) != cudaSuccess)
+    return 1;
+  return n > 0 ? n : 1;
+}
+
 template size_t tma_smem_bytes<float>();
 template size_t tma_smem_bytes<double>();
 template void launch_half_step_tma<float>(bool, const HalfStepParams<float>&, const TmaMaps&, void*);
 template void launch_half_step_tma<double>(bool, const HalfStepParams<double>&, const TmaMaps&, void*);
 template int prepare_tma_kernels<float>();
 template int prepare_tma_kernels<double>();
+template int tma_resident_ctas<float>();
+template int tma_resident_ctas<double>();
 
 }  // namespace kh
