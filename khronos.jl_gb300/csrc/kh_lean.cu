@@ -385,32 +385,40 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
 // files and for the general kernel (kh_lean.cuh says how they follow).
 template <typename T, bool H>
 __global__ void expand_state_kernel(const HalfStepParams<T> p) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.nx) return;
-  const bool f[3] = {i < p.pml_lo[0] || i >= p.nx - p.pml_hi[0], j < p.pml_lo[1] || j >= p.ny - p.pml_hi[1],
-                     k < p.pml_lo[2] || k >= p.nz - p.pml_hi[2]};
-  if (!(f[0] || f[1] || f[2])) return;
-  const long long q = p.origin + (long long)k * p.plane + (long long)j * p.pitch + i;
-  if (!KH_IN(q, p.total, 2130)) return;
-  if (p.cell_class && (p.cell_class[q] & (H ? kSpecialH : kSpecialE))) return;  // keeps the complete state
-  const int idx[3] = {i, j, k};
+  for (int k = blockIdx.z; k < p.nz; k += gridDim.z)
+    for (int j = blockIdx.y; j < p.ny; j += gridDim.y) {
+      const bool f[3] = {i < p.pml_lo[0] || i >= p.nx - p.pml_hi[0], j < p.pml_lo[1] || j >= p.ny - p.pml_hi[1],
+                         k < p.pml_lo[2] || k >= p.nz - p.pml_hi[2]};
+      if (!(f[0] || f[1] || f[2])) continue;
+      const long long q = p.origin + (long long)k * p.plane + (long long)j * p.pitch + i;
+      if (!KH_IN(q, p.total, 2130)) continue;
+      if (p.cell_class && (p.cell_class[q] & (H ? kSpecialH : kSpecialE))) continue;  // keeps the complete state
+      const int idx[3] = {i, j, k};
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const int n = (c + 1) % 3, v = (c + 2) % 3;
-    const T m = p.m_inv[c] ? p.m_inv[c][q] : p.m_scalar;
-    const T t = f[c] ? p.Ts[c][q] : (m != T(0) ? p.O[c][q] / m : T(0));
-    p.Ts[c][q] = t;
-    if (f[n] && !f[v]) p.U[c][q] = p.ax[n][idx[n]].s != T(0) ? t : T(0);
-    if (f[c]) p.W[c][q] = p.ax[c][idx[c]].s != T(0) ? mul_rn(m, t) : T(0);
-  }
+      for (int c = 0; c < 3; ++c) {
+        const int n = (c + 1) % 3, v = (c + 2) % 3;
+        const T m = p.m_inv[c] ? p.m_inv[c][q] : p.m_scalar;
+        const T t = f[c] ? p.Ts[c][q] : (m != T(0) ? p.O[c][q] / m : T(0));
+        p.Ts[c][q] = t;
+        if (f[n] && !f[v]) p.U[c][q] = p.ax[n][idx[n]].s != T(0) ? t : T(0);
+        if (f[c]) p.W[c][q] = p.ax[c][idx[c]].s != T(0) ? mul_rn(m, t) : T(0);
+      }
+    }
+}
+
+// One thread per cell; further rows and planes in turn above the grid's limits.
+template <typename T>
+static dim3 cell_grid(const HalfStepParams<T>& p) {
+  return dim3((p.nx + 127) / 128, std::min(p.ny, 65535), std::min(p.nz, 65535));
 }
 
 template <typename T>
 void launch_expand_state(bool h_half, const HalfStepParams<T>& p, void* stream) {
-  const dim3 grid((p.nx + 127) / 128, p.ny, p.nz);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (h_half) expand_state_kernel<T, true><<<grid, 128, 0, st>>>(p);
-  else expand_state_kernel<T, false><<<grid, 128, 0, st>>>(p);
+  if (h_half) expand_state_kernel<T, true><<<cell_grid(p), 128, 0, st>>>(p);
+  else expand_state_kernel<T, false><<<cell_grid(p), 128, 0, st>>>(p);
 }
 
 // What the reduced state takes for granted, checked on the complete T, U and W of a
@@ -469,10 +477,9 @@ __global__ void check_state_kernel(const HalfStepParams<T> p, StateCheck<T>* out
 
 template <typename T>
 void launch_check_state(bool h_half, const HalfStepParams<T>& p, StateCheck<T>* out, void* stream) {
-  const dim3 grid((p.nx + 127) / 128, std::min(p.ny, 65535), std::min(p.nz, 256));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (h_half) check_state_kernel<T, true><<<grid, 128, 0, st>>>(p, out);
-  else check_state_kernel<T, false><<<grid, 128, 0, st>>>(p, out);
+  if (h_half) check_state_kernel<T, true><<<cell_grid(p), 128, 0, st>>>(p, out);
+  else check_state_kernel<T, false><<<cell_grid(p), 128, 0, st>>>(p, out);
 }
 
 template <typename T, bool H, bool PV>

@@ -22,8 +22,10 @@ inline int general_zplanes(int nz, long long tiles, int slots) {
   return int(std::min<long long>(nz, std::max(2LL, std::min<long long>(10, fill))));
 }
 
-// Reduced-state kernel (kh_lean.cu).
-inline int reduced_zplanes(int nz, long long tiles, int slots, bool fp64) {
+// CTAs that a launch can have along z.
+constexpr int kMaxGridZ = 65535;
+
+inline int reduced_zplanes_by_cost(int nz, long long tiles, int slots, bool fp64) {
   // FP64 is bound by arithmetic: the shallowest chunks balance best (240×144×96, 32
   // steps: 12.26 / 12.40 / 12.50 / 12.52 / 13.0 ms at 2 / 3 / 4 / 5 / 10 planes).
   if (fp64) return std::min(2, nz);
@@ -46,6 +48,11 @@ inline int reduced_zplanes(int nz, long long tiles, int slots, bool fp64) {
     break;
   }
   return std::min(best, nz);
+}
+
+// Reduced-state kernel (kh_lean.cu).
+inline int reduced_zplanes(int nz, long long tiles, int slots, bool fp64) {
+  return std::max(reduced_zplanes_by_cost(nz, tiles, slots, fp64), (nz + kMaxGridZ - 1) / kMaxGridZ);
 }
 
 }  // namespace kh

@@ -37,3 +37,37 @@ SLOTS = 152 * 5
 def test_general_kernel_depth(plan, n, want):
     """Ten planes, or what fills two rounds of CTAs, whatever the precision."""
     assert plan.general(n[2], plan.tiles(n[0], n[1], 64, 4), SLOTS) == want
+
+
+@pytest.mark.parametrize("nz", [65535, 65536, 131070, 131071, 300000, 458746, 655350, 4000000])
+@pytest.mark.parametrize("f64", [0, 1])
+def test_reduced_kernel_depth_within_the_launch_limits(plan, nz, f64):
+    """At most 65535 CTAs along z, and at most the 64 planes a CTA has tables for."""
+    z = plan.reduced(nz, 1, 152 * 3 if f64 else 152 * 6, f64)
+    assert 1 <= z <= 64 and (nz + z - 1) // z <= 65535
+
+
+@pytest.mark.gpu
+def test_thin_column_above_the_launch_limits(kh, gpu_lib):
+    """131080 planes: two planes a CTA (FP64) would be 65540 CTAs along z, and a thread
+    block per plane 131080 in the export.  The exported state goes on bit for bit."""
+    import numpy as np
+
+    from khronos_gb300.device import GpuSim
+
+    n = (2, 2, 131080)
+    src = kh.UniformSource(time_profile=kh.GaussianPulseSource(fcen=0.8, fwidth=0.6), component=kh.EX,
+                           center=(0, 0, 0), size=(0, 0, 0))
+    sp = kh.Simulation(cell_size=tuple(a / 10 for a in n), resolution=10, sources=[src],
+                       boundaries=[[0, 0], [0, 0], [0.5, 0.5]], dtype="f64").spec()
+    assert tuple(sp.n) == n
+    a, b = GpuSim(sp, lib=gpu_lib), GpuSim(sp, lib=gpu_lib)
+    a.step(20)
+    b.import_state(a.export_state())
+    for g in (a, b):
+        g.step(10)
+        g.synchronize()
+    assert np.any(a.field(kh.EX) != 0)
+    assert np.array_equal(a.field(kh.EX), b.field(kh.EX))
+    a.close()
+    b.close()
