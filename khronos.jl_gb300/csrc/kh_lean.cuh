@@ -14,7 +14,10 @@
 // five, three instead of seven along an edge, six instead of nine in a corner.
 //
 // The operations are written with explicit roundings (no contraction left to
-// the compiler), so every kernel that uses them gives the same bits.
+// the compiler), so every kernel and every form of a row gives the same bits.  A
+// damped O is fma(m, B·d, A·O): with the factors A = B = 1 of a cell outside the
+// absorber that is the plain update, so such cells need no select (with
+// fma(A, O, m·B·d) they were rounded once more, in some forms only).
 #pragma once
 
 #include "kh_cell.cuh"
@@ -70,7 +73,7 @@ __device__ __forceinline__ void red_component(const RedAxis<T>& o, const RedAxis
       O = fma_rn(m, fma_rn(o.op, tn, -mul_rn(o.om, t)), O);
       t = tn;
     } else {
-      O = fma_rn(A, O, mul_rn(m, x));
+      O = fma_rn(m, x, mul_rn(A, O));
     }
   } else if (o.f) {
     const T tn = add_rn(t, d);
@@ -111,13 +114,13 @@ __device__ __forceinline__ void update_cells(const bool (&fx)[VN], bool anyfx, c
         const T un = fma_rn(ry.a, u.c[0].v[v], mul_rn(ry.b, K.c[0].v[v]));
         const T d = sub_rn(un, u.c[0].v[v]);
         u.c[0].v[v] = un;
-        O.c[0].v[v] = fma_rn(rz.a, O.c[0].v[v], mul_rn(m.c[0].v[v], mul_rn(rz.b, d)));
+        O.c[0].v[v] = fma_rn(m.c[0].v[v], mul_rn(rz.b, d), mul_rn(rz.a, O.c[0].v[v]));
       }
     } else {
       const T A = ry.f ? ry.a : rz.a, B = ry.f ? ry.b : rz.b;
 #pragma unroll
       for (int v = 0; v < VN; ++v)
-        O.c[0].v[v] = fma_rn(A, O.c[0].v[v], mul_rn(m.c[0].v[v], mul_rn(B, K.c[0].v[v])));
+        O.c[0].v[v] = fma_rn(m.c[0].v[v], mul_rn(B, K.c[0].v[v]), mul_rn(A, O.c[0].v[v]));
     }
     // component y: own axis y, damped along z; component z the other way
 #pragma unroll
@@ -134,7 +137,7 @@ __device__ __forceinline__ void update_cells(const bool (&fx)[VN], bool anyfx, c
       } else {
 #pragma unroll
         for (int v = 0; v < VN; ++v)
-          O.c[c].v[v] = fma_rn(d.a, O.c[c].v[v], mul_rn(m.c[c].v[v], mul_rn(d.b, K.c[c].v[v])));
+          O.c[c].v[v] = fma_rn(m.c[c].v[v], mul_rn(d.b, K.c[c].v[v]), mul_rn(d.a, O.c[c].v[v]));
       }
     }
   } else if (!(ry.f || rz.f)) {
@@ -143,11 +146,9 @@ __device__ __forceinline__ void update_cells(const bool (&fx)[VN], bool anyfx, c
       const AxisCoef<T> x = xt[v];  // a, b, 1-σ, 1+σ
       const T tn = add_rn(t.c[0].v[v], K.c[0].v[v]);
       const T o0 = fma_rn(m.c[0].v[v], fma_rn(x.op, tn, -mul_rn(x.ir, t.c[0].v[v])), O.c[0].v[v]);
-      const T o1 = fma_rn(x.s, O.c[1].v[v], mul_rn(m.c[1].v[v], mul_rn(x.om, K.c[1].v[v])));
-      const T o2 = fma_rn(x.s, O.c[2].v[v], mul_rn(m.c[2].v[v], mul_rn(x.om, K.c[2].v[v])));
       O.c[0].v[v] = fx[v] ? o0 : fma_rn(m.c[0].v[v], K.c[0].v[v], O.c[0].v[v]);
-      O.c[1].v[v] = fx[v] ? o1 : fma_rn(m.c[1].v[v], K.c[1].v[v], O.c[1].v[v]);
-      O.c[2].v[v] = fx[v] ? o2 : fma_rn(m.c[2].v[v], K.c[2].v[v], O.c[2].v[v]);
+      O.c[1].v[v] = fma_rn(m.c[1].v[v], mul_rn(x.om, K.c[1].v[v]), mul_rn(x.s, O.c[1].v[v]));
+      O.c[2].v[v] = fma_rn(m.c[2].v[v], mul_rn(x.om, K.c[2].v[v]), mul_rn(x.s, O.c[2].v[v]));
       t.c[0].v[v] = fx[v] ? tn : t.c[0].v[v];
     }
   } else {
@@ -193,7 +194,7 @@ __device__ __forceinline__ void update_row(const bool (&fx)[VN], const AxisCoef<
       const T A = FZ ? za : ry.a, B = FZ ? zb : ry.b;
       const T w = FY || FZ ? mul_rn(B, d) : d;
       const T o = O.c[0].v[v], mm = m.c[0].v[v], tt = t.c[0].v[v];
-      T r = FY || FZ ? fma_rn(A, o, mul_rn(mm, w)) : fma_rn(mm, w, o);
+      T r = FY || FZ ? fma_rn(mm, w, mul_rn(A, o)) : fma_rn(mm, w, o);
       if constexpr (WX) {
         const T tn = FY || FZ ? fma_rn(A, tt, w) : add_rn(tt, w);
         const T rt = fma_rn(mm, fma_rn(x.op, tn, -mul_rn(x.ir, tt)), o);
@@ -222,7 +223,7 @@ __device__ __forceinline__ void update_row(const bool (&fx)[VN], const AxisCoef<
         O.c[1].v[v] = fma_rn(mm, fma_rn(ry.op, tn, -mul_rn(ry.om, tt)), o);
         t.c[1].v[v] = tn;
       } else {
-        O.c[1].v[v] = damp ? fma_rn(A, o, mul_rn(mm, w)) : fma_rn(mm, w, o);
+        O.c[1].v[v] = fma_rn(mm, w, damp ? mul_rn(A, o) : o);
       }
     }
     {  // component z: own axis z, next x, previous y
@@ -244,7 +245,7 @@ __device__ __forceinline__ void update_row(const bool (&fx)[VN], const AxisCoef<
         O.c[2].v[v] = fma_rn(mm, fma_rn(zop, tn, -mul_rn(zom, tt)), o);
         t.c[2].v[v] = tn;
       } else {
-        O.c[2].v[v] = damp ? fma_rn(A, o, mul_rn(mm, w)) : fma_rn(mm, w, o);
+        O.c[2].v[v] = fma_rn(mm, w, damp ? mul_rn(A, o) : o);
       }
     }
   }
