@@ -53,7 +53,7 @@ struct FusedGeom {
 }  // namespace
 
 template <typename T, bool PV>
-__global__ void __launch_bounds__(32 * kFusedRows, kFusedMinBlocks)
+__global__ void __launch_bounds__(32 * kFusedRows, PV ? kFusedMinBlocks : kFusedMinBlocks + 1)
     step_fused_kernel(const __grid_constant__ FusedParams<T> p, const __grid_constant__ FusedMaps maps) {
   using G = FusedGeom<T, PV>;
   constexpr int VN = 2;
@@ -143,6 +143,16 @@ __global__ void __launch_bounds__(32 * kFusedRows, kFusedMinBlocks)
   for (int l = l0; l <= N; ++l) {
     const int sn = st + 1 == kFusedStages ? 0 : st + 1;
     const uint32_t pn = sn == 0 ? parity ^ 1u : parity;
+    // special rows: class words and D on their way together, before the wait and the
+    // H update, instead of one after the other between the plane's two barriers
+    const bool tf = own && l > 0 && (tbits & 1ull);
+    uint2 cls{0u, 0u};
+    Cells<T, VN> D;
+    if (tf && KH_IN(q, p.total, 2227) && KH_IN(q + VN - 1, p.total, 2227)) {
+      cls = *reinterpret_cast<const uint2*>(p.cell_class + q);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) D.c[c] = *reinterpret_cast<const PK*>(p.D[c] + q);
+    }
     if (gave_up < 0 && !mbar_wait_sleep(smem_u32(bars + sn), pn, kSleepWaitLimit)) {
       gave_up = l;
       if (p.err) atomicExch(p.err, KH_ERR_TIMEOUT);
@@ -206,7 +216,7 @@ __global__ void __launch_bounds__(32 * kFusedRows, kFusedMinBlocks)
           for (int v = 0; v < VN; ++v) m.c[c].v[v] = p.eps_scalar;
         }
       }
-      if (!(tbits & 1ull)) {
+      if (!tf) {
 #pragma unroll
         for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -214,12 +224,11 @@ __global__ void __launch_bounds__(32 * kFusedRows, kFusedMinBlocks)
       } else {
 #pragma unroll
         for (int v = 0; v < VN; ++v) {
-          const bool sp =
-              x0 + v < p.nx && KH_IN(q + v, p.total, 2227) && (p.cell_class[q + v] & kSpecialE) != 0;
+          const bool sp = x0 + v < p.nx && ((v ? cls.y : cls.x) & kSpecialE) != 0;
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             if (sp) {  // keeps its D state
-              const T t = add_rn(p.D[c][q + v], K.c[c].v[v]);
+              const T t = add_rn(D.c[c].v[v], K.c[c].v[v]);
               p.D[c][q + v] = t;
               E.c[c].v[v] = mul_rn(m.c[c].v[v], t);
             } else {

@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
     half_step_lean_kernel(const __grid_constant__ HalfStepParams<T> p, const __grid_constant__ TmaMaps maps) {
   using G = LeanGeom<T, PV>;
   constexpr int VN = kLeanVN;
+  static_assert(VN == 2, "paired loads of the class words");
   // Rows in update_row's branch-free forms, except in FP32 with per-voxel m⁻¹, where
   // their longer live ranges spill at six CTAs per SM (320×192×128, 96 steps: 15.96 ms
   // with update_cells in both halves, 15.37 with this choice, 15.73 with update_row in
@@ -204,7 +205,15 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
     // with special cells take all of them
     Cells<T, VN> t, u;
     if constexpr (kRow) t = u = Cells<T, VN>{};
+    uint2 cls{0u, 0u};  // class words of the two cells
+    auto read_cls = [&] {
+      if (KH_IN(q, p.total, 2110) && KH_IN(q + VN - 1, p.total, 2110))
+        cls = *reinterpret_cast<const uint2*>(p.cell_class + q);
+    };
     if (!plain && lane_ok) {
+      // FP64 reads them with the auxiliaries; in FP32 their registers cost the rows
+      // without special cells more (320×192×128, 96 steps: 14.97 to 15.12 ms)
+      if (sizeof(T) == 8 && tf) read_cls();
       if (anyfx || tf) t.c[0] = get(p.Ts[0], 2104);
       if (fy || tf) t.c[1] = get(p.Ts[1], 2105);
       if (fz || tf) t.c[2] = get(p.Ts[2], 2106);
@@ -261,9 +270,10 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
       bool sp[VN], anysp = false;
       if (tf) {
         constexpr uint32_t kSp = H ? kSpecialH : kSpecialE;
+        if (sizeof(T) == 4) read_cls();
 #pragma unroll
         for (int v = 0; v < VN; ++v) {
-          sp[v] = x0 + v < p.nx && KH_IN(q + v, p.total, 2110) && (p.cell_class[q + v] & kSp) != 0;
+          sp[v] = x0 + v < p.nx && ((v ? cls.y : cls.x) & kSp) != 0;
           anysp |= sp[v];
         }
       }
