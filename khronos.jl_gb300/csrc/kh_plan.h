@@ -25,10 +25,39 @@ inline int general_zplanes(int nz, long long tiles, int slots) {
 // CTAs that a launch can have along z.
 constexpr int kMaxGridZ = 65535;
 
-inline int reduced_zplanes_by_cost(int nz, long long tiles, int slots, bool fp64) {
-  // FP64 is bound by arithmetic: the shallowest chunks balance best (240×144×96, 32
-  // steps: 12.26 / 12.40 / 12.50 / 12.52 / 13.0 ms at 2 / 3 / 4 / 5 / 10 planes).
-  if (fp64) return std::min(2, nz);
+// Time of a launch of FP64 chunks of z planes, in planes of a full SM: bound by
+// arithmetic, so a round of resident CTAs takes its planes times its CTAs per SM, a
+// CTA alone on its SM 1.4 times its share; a CTA's start costs 0.3 planes.
+inline double reduced_cost_f64(int nz, long long tiles, int slots, int sms, int z) {
+  const long long ctas = tiles * ((nz + z - 1) / z), rounds = ctas / slots;
+  const int per_sm = std::max(1, slots / sms), last = int((ctas % slots + sms - 1) / sms);
+  return (z + 0.3) * (double(rounds * per_sm) + (last == 0 ? 0.0 : std::max(1.4, double(last))));
+}
+
+inline int reduced_zplanes_f64(int nz, long long tiles, int slots, int sms, bool cpml) {
+  // Without CPML all planes cost the same and deeper chunks save starts and halo
+  // planes.  With it, chunks of two balance the planes inside and outside best, unless
+  // their last round of CTAs is nearly empty.  Another depth than two has to promise
+  // more than the estimate is off by.  µs a step at 2 / 3 / 4 / 5 / 6 planes, without
+  // CPML: 64³ 35.7 / 36.7 / 32.3 / 37.2 / 41.5, 100³ 104 / 100 / 98 / 119 / 97, 181×97×75 113 /
+  // 119 / 116 / 122 / 115, 240×144×96 265 / 257 / 259 / 248 / 267, 320×192×128 561 / 541 /
+  // 539 / 532 / 523; with: 64³ 54.5 / 56.1 / 52.9 / 62.1 / 75.0, 100³ 155 / 160 / 166 / 178 /
+  // 166, 181×97×75 157 / 164 / 165 / 180 / 182, 240×144×96 333 / 334 / 336 / 338 / 348,
+  // 320×192×128 655 / 645 / 652 / 644 / 650.
+  int best = std::min(2, nz);
+  const double two = reduced_cost_f64(nz, tiles, slots, sms, best);
+  double least = (cpml ? 0.9 : 0.95) * two;
+  for (int z = 3; z <= std::min(6, nz); ++z) {
+    const double c = reduced_cost_f64(nz, tiles, slots, sms, z);
+    if (c < least) {
+      least = c;
+      best = z;
+    }
+  }
+  return best;
+}
+
+inline int reduced_zplanes_f32(int nz, long long tiles, int slots) {
   // A plane costs a CTA about 1.4 µs whatever else runs, its start about three
   // planes; more rounds of CTAs cost less than their number (the SMs overlap them).
   // The optimum of that grows with the square root of the rounds at one plane per
@@ -51,8 +80,9 @@ inline int reduced_zplanes_by_cost(int nz, long long tiles, int slots, bool fp64
 }
 
 // Reduced-state kernel (kh_lean.cu).
-inline int reduced_zplanes(int nz, long long tiles, int slots, bool fp64) {
-  return std::max(reduced_zplanes_by_cost(nz, tiles, slots, fp64), (nz + kMaxGridZ - 1) / kMaxGridZ);
+inline int reduced_zplanes(int nz, long long tiles, int slots, int sms, bool fp64, bool cpml) {
+  const int z = fp64 ? reduced_zplanes_f64(nz, tiles, slots, sms, cpml) : reduced_zplanes_f32(nz, tiles, slots);
+  return std::max(z, (nz + kMaxGridZ - 1) / kMaxGridZ);
 }
 
 }  // namespace kh

@@ -1958,11 +1958,10 @@ class Sim : public SimBase {
         return fail(KH_ERR_CUDA, "cudaFuncSetAttribute on the whole-step kernels failed");
       attr_done[dev] = true;
     }
-    int sms = 0;
-    KH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (sizeof(T) == 4) fused_slots_ = sms * kh::fused_resident_ctas<float>();
-    lean_slots_ = sms * kh::lean_resident_ctas<T>();
-    tma_slots_ = sms * kh::tma_resident_ctas<T>();
+    KH_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
+    if (sizeof(T) == 4) fused_slots_ = sms_ * kh::fused_resident_ctas<float>();
+    lean_slots_ = sms_ * kh::lean_resident_ctas<T>();
+    tma_slots_ = sms_ * kh::tma_resident_ctas<T>();
     const int hx = 16 / int(sizeof(T));
     struct MapSet {
       kh::TmaMaps *h, *e;
@@ -1998,7 +1997,8 @@ class Sim : public SimBase {
   void choose_zplanes() {
     zplanes_ = general_zplanes_ = std::min(10, n_[2]);
     if (use_tma_) {
-      zplanes_ = kh::reduced_zplanes(n_[2], kh::plan_tiles(n_[0], n_[1], kh::kLeanX, kh::kLeanY), lean_slots_, sizeof(T) == 8);
+      zplanes_ = kh::reduced_zplanes(n_[2], kh::plan_tiles(n_[0], n_[1], kh::kLeanX, kh::kLeanY), lean_slots_, sms_,
+                                     sizeof(T) == 8, pml_axis_[0] || pml_axis_[1] || pml_axis_[2]);
       general_zplanes_ = kh::general_zplanes(n_[2], kh::plan_tiles(n_[0], n_[1], kh::kTmaX, kh::kTmaY), tma_slots_);
     }
     if (const char* zv = std::getenv("KHRONOS_GB300_ZPLANES")) {
@@ -2373,6 +2373,7 @@ class Sim : public SimBase {
   int zplanes_ = 10, general_zplanes_ = 10;  // of kh_lean.cu, of kh_tma.cu
   int xprefetch_ = 2;        // x-CPML state prefetch mode (HalfStepParams::xprefetch)
   int xpf_dist_ = 3;
+  int sms_ = 1;
   int fused_slots_ = 1;  // SMs × resident whole-step CTAs per SM
   int lean_slots_ = 1, tma_slots_ = 1;  // … reduced-state, general-kernel CTAs per SM
   kh::TmaMaps maps_h_, maps_e_;            // kTmaY rows (general kernel)

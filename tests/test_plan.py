@@ -11,7 +11,9 @@ WRAP = """
 extern "C" {
 long long tiles(int nx, int ny, int tx, int ty) { return kh::plan_tiles(nx, ny, tx, ty); }
 int general(int nz, long long t, int s) { return kh::general_zplanes(nz, t, s); }
-int reduced(int nz, long long t, int s, int f64) { return kh::reduced_zplanes(nz, t, s, f64 != 0); }
+int reduced(int nz, long long t, int s, int sms, int f64, int cpml) {
+  return kh::reduced_zplanes(nz, t, s, sms, f64 != 0, cpml != 0);
+}
 }
 """
 
@@ -25,7 +27,7 @@ def plan(tmp_path_factory):
     lib = C.CDLL(str(d / "plan.so"))
     lib.tiles.restype = C.c_longlong
     lib.general.argtypes = [C.c_int, C.c_longlong, C.c_int]
-    lib.reduced.argtypes = [C.c_int, C.c_longlong, C.c_int, C.c_int]
+    lib.reduced.argtypes = [C.c_int, C.c_longlong, C.c_int, C.c_int, C.c_int, C.c_int]
     return lib
 
 
@@ -43,8 +45,21 @@ def test_general_kernel_depth(plan, n, want):
 @pytest.mark.parametrize("f64", [0, 1])
 def test_reduced_kernel_depth_within_the_launch_limits(plan, nz, f64):
     """At most 65535 CTAs along z, and at most the 64 planes a CTA has tables for."""
-    z = plan.reduced(nz, 1, 152 * 3 if f64 else 152 * 6, f64)
+    z = plan.reduced(nz, 1, 152 * 3 if f64 else 152 * 6, 152, f64, 1)
     assert 1 <= z <= 64 and (nz + z - 1) // z <= 65535
+
+
+@pytest.mark.parametrize("n,open_box,cpml", [((48, 48, 48), (2,), (2,)), ((64, 64, 64), (4,), (2, 3, 4)),
+                                             ((100, 100, 100), (2, 3, 4, 6), (2, 3, 4, 6)),
+                                             ((181, 97, 75), (2, 3, 4, 6), (2, 3, 4)),
+                                             ((240, 144, 96), (2, 3, 4, 5, 6), (2, 3, 4, 5, 6)),
+                                             ((320, 192, 128), (2, 3, 4, 5, 6), (2, 3, 4, 5, 6)),
+                                             ((20, 20, 1), (1,), (1,))])
+def test_fp64_depth(plan, n, open_box, cpml):
+    """One of the depths measured within 8 % of the fastest (the figures beside the rule)."""
+    t = plan.tiles(n[0], n[1], 64, 4)
+    assert plan.reduced(n[2], t, 152 * 3, 152, 1, 0) in open_box
+    assert plan.reduced(n[2], t, 152 * 3, 152, 1, 1) in cpml
 
 
 @pytest.mark.gpu
