@@ -136,6 +136,10 @@ struct alignas(16) SlotPack {
   Cplx<T> amp;   // complex amplitude
 };
 
+// HalfStepParams::view, in CPML cells outside the own-axis CPML: O from its copy in the
+// array of T, the copy from O.
+constexpr uint32_t kViewRestore = 1u, kViewKeep = 2u;
+
 // Parameters of one fused half-step launch.
 template <typename T>
 struct HalfStepParams {
@@ -161,6 +165,10 @@ struct HalfStepParams {
   const T* msig[3];   // material conductivity σB / σD or nullptr
   const AxisCoef<T>* ax[3];  // CPML coefficients per axis at cell centres (length n_a)
   int pml_lo[3], pml_hi[3];
+  // the same without the layers of σ = 0 at the inner edge, which damp nothing: what the
+  // reduced-state kernel takes for its CPML
+  int red_lo[3], red_hi[3];
+  __host__ __device__ int n_axis(int a) const { return a == 0 ? nx : (a == 1 ? ny : nz); }
   int cpml;                    // 1: CUDA-path CPML stages, 0: CPU-path dispatch
   uint32_t sigma_region_mask;  // bit r (r = rx + 3 ry + 9 rz) set: region has conductivity
 
@@ -191,6 +199,10 @@ struct HalfStepParams {
   // the same mask for the reduced-state kernel, which writes the ghost layers of
   // its half itself
   uint32_t wrap;
+  // reduced-state kernel, while the program holds views of the fields: kViewRestore
+  // in the first step of a call, kViewKeep in the last one
+  uint32_t view;
+  int view_form;  // 2: the form for grids of more than one round of CTAs
 
   int* err;  // set to KH_ERR_TIMEOUT by a kernel whose bounded wait gave up
   // Failure-detection test hook (0 in normal runs): nonzero launches the FP32
@@ -329,11 +341,38 @@ template <typename T>
 int tma_resident_ctas();
 
 // Reduced-state half-step (kh_lean.cu) for the CUDA-path CPML stages; its maps
-// have boxes of kLeanY rows.  expand: the complete T, U, W from its state.
+// have boxes of kLeanY rows.  expand: the complete T, U, W from its state (o_kept: the
+// array of T holds a copy of O where O is the state, see KeepArgs).
 template <typename T>
 void launch_half_step_lean(bool h_half, const HalfStepParams<T>& p, const TmaMaps& maps, void* stream);
 template <typename T>
-void launch_expand_state(bool h_half, const HalfStepParams<T>& p, void* stream);
+void launch_expand_state(bool h_half, const HalfStepParams<T>& p, bool o_kept, void* stream);
+// While the program holds views of the fields: in CPML cells outside the own-axis CPML O
+// is the state, but a value written there through a view is not to stay (as where D is
+// kept).  Between calls the array of T, free there, holds a copy of O, which the steps at
+// both ends of a call mind (HalfStepParams::view).  This makes the copies outside of a
+// step; from_t: out of the complete state.
+template <typename T>
+struct KeepHalf {
+  T *O[3], *Ts[3];
+  const T* m_inv[3];
+  T m_scalar;
+  int lo[3], hi[3];  // HalfStepParams::red_lo, red_hi
+  const uint64_t* tile_bits;
+  uint32_t special;  // its class bit
+};
+template <typename T>
+struct KeepArgs {
+  KeepHalf<T> half[2];
+  int n[3], nxb;
+  long long pitch, plane, origin, total;
+  const uint32_t* cell_class;
+  // the layers as six boxes that do not overlap; prefix sums of their cells
+  int start[6][3], dims[6][3];
+  long long first[7];
+};
+template <typename T>
+void launch_keep_state(const KeepArgs<T>& a, int halves, bool from_t, void* stream);
 // A complete state against what the reduced one takes for granted in CPML cells
 // without special state: broken, W = m·T (own axis) or O = m·T (outside it) does not
 // hold to rounding; off_u against top_t, the largest |U - T| where only the next axis
@@ -348,9 +387,10 @@ template <typename T>
 void launch_check_state(bool h_half, const HalfStepParams<T>& p, StateCheck<T>* out, void* stream);
 template <typename T>
 int prepare_lean_kernels();
-// CTAs of the reduced-state kernel resident on one SM (after prepare).
+// CTAs of the reduced-state kernel (view: HalfStepParams::view_form) resident on one
+// SM (after prepare).
 template <typename T>
-int lean_resident_ctas();
+int lean_resident_ctas(int view);
 
 // History recording: the components of up to kMaxRecords monitors over their cell
 // boxes (x fastest) into a contiguous slot of each one's history buffer, in one launch.

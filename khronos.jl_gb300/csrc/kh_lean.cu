@@ -53,8 +53,18 @@ struct LeanGeom {
 
 constexpr int kLeanThreads = kLeanY * kLeanX / kLeanVN;
 
-template <typename T, bool H, bool PV, bool STALL = false, bool PER = false>
-__global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
+// VIEW: the first or last step of a call while the program holds views of this half's
+// fields (HalfStepParams::view).  In the absorber outside the own-axis CPML O is the
+// state, but a value written through a view does not belong to it; the array of T, free
+// there, holds a copy of O between calls.  Such a step moves as much as the complete
+// cascade does.  In FP32 with per-voxel m⁻¹ it spills at six CTAs per SM (VIEW 1), which
+// small grids, all of them resident at once, bear better than fewer CTAs; others take
+// five (VIEW 2).  µs a step of calls of one step, 64³ / 96³ / 160×160×96, where the copies
+// no longer fit the L2: without views 26.3 / 42.5 / 75, VIEW 1 31.6 / 49.2 / 102, VIEW 2
+// 31.0 / 54.3 / 93.5, the complete cascade 30.7 / 56.2 / 94.8, the copies in launches of
+// their own 39.7 / 59.9 / 117.
+template <typename T, bool H, bool PV, bool STALL = false, bool PER = false, int VIEW = 0>
+__global__ void __launch_bounds__(kLeanThreads, (VIEW == 2 ? kLeanMinBlocks<T> - 1 : kLeanMinBlocks<T>))
     half_step_lean_kernel(const __grid_constant__ HalfStepParams<T> p, const __grid_constant__ TmaMaps maps) {
   using G = LeanGeom<T, PV>;
   constexpr int VN = kLeanVN;
@@ -87,8 +97,8 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
   const int k1 = min(k0 + p.zplanes, p.nz);
   const int N = k1 - k0;
   constexpr int kLimit = STALL ? kStallSleepWaitLimit : kSleepWaitLimit;
-  const bool tfx = x_tile < p.pml_lo[0] || (p.pml_hi[0] > 0 && x_tile + kLeanX > p.nx - p.pml_hi[0]);
-  const bool tfy = y_tile < p.pml_lo[1] || (p.pml_hi[1] > 0 && y_tile + kLeanY > p.ny - p.pml_hi[1]);
+  const bool tfx = x_tile < p.red_lo[0] || (p.red_hi[0] > 0 && x_tile + kLeanX > p.nx - p.red_hi[0]);
+  const bool tfy = y_tile < p.red_lo[1] || (p.red_hi[1] > 0 && y_tile + kLeanY > p.ny - p.red_hi[1]);
 
   if (issuer) {
     for (int st = 0; st < kLeanStages; ++st) mbar_init(&bars[st], 1);
@@ -97,13 +107,13 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
   if (tfx)
     for (int c = tid; c < kLeanX; c += kLeanThreads) {
       const int i = x_tile + c;
-      const bool f = i < p.nx && (i < p.pml_lo[0] || i >= p.nx - p.pml_hi[0]);
+      const bool f = i < p.nx && (i < p.red_lo[0] || i >= p.nx - p.red_hi[0]);
       const RedAxis<T> r = red_axis<T>(f && KH_IN(i, p.nx, 2120) ? p.ax[0][i] : AxisCoef<T>{}, f);
       xtab[c] = {r.a, r.b, r.om, r.op};
     }
-  if (k0 < p.pml_lo[2] || k1 > p.nz - p.pml_hi[2])
+  if (k0 < p.red_lo[2] || k1 > p.nz - p.red_hi[2])
     for (int c = tid; c < N; c += kLeanThreads) {
-      const bool f = k0 + c < p.pml_lo[2] || k0 + c >= p.nz - p.pml_hi[2];
+      const bool f = k0 + c < p.red_lo[2] || k0 + c >= p.nz - p.red_hi[2];
       const RedAxis<T> r = red_axis<T>(f && KH_IN(k0 + c, p.nz, 2112) ? p.ax[2][k0 + c] : AxisCoef<T>{}, f);
       ztab[c] = {r.a, r.b, r.om, r.op};
     }
@@ -134,7 +144,7 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
     }
     // the plane's y/z auxiliaries into L2 ahead of the register loads (the
     // x ones, a few columns of the tile, are fetched by their own lanes)
-    const bool tfz = k < p.pml_lo[2] || k >= p.nz - p.pml_hi[2];
+    const bool tfz = k < p.red_lo[2] || k >= p.nz - p.red_hi[2];
     if (tfy) tma_prefetch_3d(&maps.t[1], G::XO + x_tile, 1 + y_tile, zc);
     if (tfz) tma_prefetch_3d(&maps.t[2], G::XO + x_tile, 1 + y_tile, zc);
     if (tfy && tfz) tma_prefetch_3d(&maps.u[0], G::XO + x_tile, 1 + y_tile, zc);
@@ -168,14 +178,25 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
       nb1 = *reinterpret_cast<const PK*>(p.A[1] + qn);
     }
   }
-  const bool fy = lane_ok && (j < p.pml_lo[1] || j >= p.ny - p.pml_hi[1]);
+  const bool fy = lane_ok && (j < p.red_lo[1] || j >= p.ny - p.red_hi[1]);
   const RedAxis<T> ry = red_axis<T>(fy && KH_IN(j, p.ny, 2111) ? p.ax[1][j] : AxisCoef<T>{}, fy);
   bool fxv[VN], anyfx = false;
 #pragma unroll
   for (int v = 0; v < VN; ++v) {
     const int i = x0 + v;
-    fxv[v] = tfx && lane_ok && i < p.nx && (i < p.pml_lo[0] || i >= p.nx - p.pml_hi[0]);
+    fxv[v] = tfx && lane_ok && i < p.nx && (i < p.red_lo[0] || i >= p.nx - p.red_hi[0]);
     anyfx |= fxv[v];
+  }
+  // VIEW: the absorber's layers with those of σ = 0
+  auto in_layer = [&](int a, int i) { return i < p.pml_lo[a] || i >= p.n_axis(a) - p.pml_hi[a]; };
+  bool lxv[VN] = {}, ly = false, anylx = false;
+  if constexpr (VIEW != 0) {
+#pragma unroll
+    for (int v = 0; v < VN; ++v) {
+      lxv[v] = lane_ok && x0 + v < p.nx && in_layer(0, x0 + v);
+      anylx |= lxv[v];
+    }
+    ly = lane_ok && in_layer(1, j);
   }
   // special-cell plane bits of this row segment, one word per 64 planes
   const long long tb_group = (long long)p.ny * p.nxb;
@@ -198,25 +219,27 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
   int st = 0;        // ring stage of load n, and the parity of its phase
   uint32_t parity = 0;
   for (int n = 0; n < N; ++n) {
-    const bool fz = k < p.pml_lo[2] || k >= p.nz - p.pml_hi[2];
+    const bool fz = k < p.red_lo[2] || k >= p.nz - p.red_hi[2];
     const bool tf = H ? (tbits >> 63) != 0 : (tbits & 1ull) != 0;
     const bool plain = !(anyfx || fy || fz || tf);
+    const bool lz = VIEW != 0 && in_layer(2, k), layer = VIEW != 0 && (anylx || ly || lz);
+    const bool all_t = tf || layer;
     // auxiliaries: T in the own-axis CPML, U in those of both other axes; rows
-    // with special cells take all of them
+    // with special cells take all of them, VIEW steps all of T
     Cells<T, VN> t, u;
-    if constexpr (kRow) t = u = Cells<T, VN>{};
+    if constexpr (kRow || VIEW != 0) t = u = Cells<T, VN>{};
     uint2 cls{0u, 0u};  // class words of the two cells
     auto read_cls = [&] {
       if (KH_IN(q, p.total, 2110) && KH_IN(q + VN - 1, p.total, 2110))
         cls = *reinterpret_cast<const uint2*>(p.cell_class + q);
     };
-    if (!plain && lane_ok) {
+    if ((!plain || layer) && lane_ok) {
       // FP64 reads them with the auxiliaries; in FP32 their registers cost the rows
       // without special cells more (320×192×128, 96 steps: 14.97 to 15.12 ms)
       if (sizeof(T) == 8 && tf) read_cls();
-      if (anyfx || tf) t.c[0] = get(p.Ts[0], 2104);
-      if (fy || tf) t.c[1] = get(p.Ts[1], 2105);
-      if (fz || tf) t.c[2] = get(p.Ts[2], 2106);
+      if (anyfx || all_t) t.c[0] = get(p.Ts[0], 2104);
+      if (fy || all_t) t.c[1] = get(p.Ts[1], 2105);
+      if (fz || all_t) t.c[2] = get(p.Ts[2], 2106);
       if (fy && (fz || tf)) u.c[0] = get(p.U[0], 2107);
       if (fz && (anyfx || tf)) u.c[1] = get(p.U[1], 2108);
       if (anyfx && (fy || tf)) u.c[2] = get(p.U[2], 2109);
@@ -267,7 +290,7 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
       nb0 = c0;
       nb1 = c1;
       const AxisCoef<T> zt = ztab[k - k0];  // read where fz
-      bool sp[VN], anysp = false;
+      bool sp[VN] = {}, anysp = false;
       if (tf) {
         constexpr uint32_t kSp = H ? kSpecialH : kSpecialE;
         if (sizeof(T) == 4) read_cls();
@@ -275,6 +298,19 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
         for (int v = 0; v < VN; ++v) {
           sp[v] = x0 + v < p.nx && ((v ? cls.y : cls.x) & kSp) != 0;
           anysp |= sp[v];
+        }
+      }
+      // O is the state: a cell of a layer, outside the own-axis CPML
+      auto derived = [&](int c, int v) {
+        return (lxv[v] || ly || lz) && !(c == 0 ? fxv[v] : (c == 1 ? fy : fz)) && !sp[v];
+      };
+      if constexpr (VIEW != 0) {
+        if (p.view & kViewRestore) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int v = 0; v < VN; ++v)
+              if (derived(c, v)) O.c[c].v[v] = t.c[c].v[v];
         }
       }
       if (anysp) {
@@ -315,11 +351,20 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
           }
         }
       }
-      if (!plain) {
+      if constexpr (VIEW != 0) {
+        if (p.view & kViewKeep) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int v = 0; v < VN; ++v)
+              if (derived(c, v)) t.c[c].v[v] = O.c[c].v[v];
+        }
+      }
+      if (!plain || layer) {
         // what was loaded goes back (values that a cell does not use unchanged)
-        if (anyfx || tf) put(p.Ts[0] + q, t.c[0], 2121);
-        if (fy || tf) put(p.Ts[1] + q, t.c[1], 2122);
-        if (fz || tf) put(p.Ts[2] + q, t.c[2], 2123);
+        if (anyfx || all_t) put(p.Ts[0] + q, t.c[0], 2121);
+        if (fy || all_t) put(p.Ts[1] + q, t.c[1], 2122);
+        if (fz || all_t) put(p.Ts[2] + q, t.c[2], 2123);
         if (fy && (fz || tf)) put(p.U[0] + q, u.c[0], 2124);
         if (fz && (anyfx || tf)) put(p.U[1] + q, u.c[1], 2125);
         if (anyfx && (fy || tf)) put(p.U[2] + q, u.c[2], 2126);
@@ -391,17 +436,30 @@ __global__ void __launch_bounds__(kLeanThreads, (kLeanMinBlocks<T>))
 }
 
 // ---------------------------------------------------------------------------
+// The CPML axes of a cell (layers of σ = 0 at its inner edge count as outside); whether
+// it lies in a layer at all, where the complete state has T.
+template <typename T>
+__device__ __forceinline__ bool in_absorber(const HalfStepParams<T>& p, int i, int j, int k, bool (&f)[3]) {
+  const int at[3] = {i, j, k};
+  bool any = false;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    f[a] = at[a] < p.red_lo[a] || at[a] >= p.n_axis(a) - p.red_hi[a];
+    any |= at[a] < p.pml_lo[a] || at[a] >= p.n_axis(a) - p.pml_hi[a];
+  }
+  return any;
+}
+
 // The complete T, U, W of every CPML cell from the reduced state, for state
 // files and for the general kernel (kh_lean.cuh says how they follow).
 template <typename T, bool H>
-__global__ void expand_state_kernel(const HalfStepParams<T> p) {
+__global__ void expand_state_kernel(const HalfStepParams<T> p, bool o_kept) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.nx) return;
   for (int k = blockIdx.z; k < p.nz; k += gridDim.z)
     for (int j = blockIdx.y; j < p.ny; j += gridDim.y) {
-      const bool f[3] = {i < p.pml_lo[0] || i >= p.nx - p.pml_hi[0], j < p.pml_lo[1] || j >= p.ny - p.pml_hi[1],
-                         k < p.pml_lo[2] || k >= p.nz - p.pml_hi[2]};
-      if (!(f[0] || f[1] || f[2])) continue;
+      bool f[3];
+      if (!in_absorber(p, i, j, k, f)) continue;
       const long long q = p.origin + (long long)k * p.plane + (long long)j * p.pitch + i;
       if (!KH_IN(q, p.total, 2130)) continue;
       if (p.cell_class && (p.cell_class[q] & (H ? kSpecialH : kSpecialE))) continue;  // keeps the complete state
@@ -410,10 +468,10 @@ __global__ void expand_state_kernel(const HalfStepParams<T> p) {
       for (int c = 0; c < 3; ++c) {
         const int n = (c + 1) % 3, v = (c + 2) % 3;
         const T m = p.m_inv[c] ? p.m_inv[c][q] : p.m_scalar;
-        const T t = f[c] ? p.Ts[c][q] : (m != T(0) ? p.O[c][q] / m : T(0));
+        const T t = f[c] ? p.Ts[c][q] : derived_t(o_kept ? p.Ts[c][q] : p.O[c][q], m);
         p.Ts[c][q] = t;
-        if (f[n] && !f[v]) p.U[c][q] = p.ax[n][idx[n]].s != T(0) ? t : T(0);
-        if (f[c]) p.W[c][q] = p.ax[c][idx[c]].s != T(0) ? mul_rn(m, t) : T(0);
+        if (f[n] && !f[v] && p.ax[n][idx[n]].s != T(0)) p.U[c][q] = t;
+        if (f[c] && p.ax[c][idx[c]].s != T(0)) p.W[c][q] = mul_rn(m, t);
       }
     }
 }
@@ -425,10 +483,58 @@ static dim3 cell_grid(const HalfStepParams<T>& p) {
 }
 
 template <typename T>
-void launch_expand_state(bool h_half, const HalfStepParams<T>& p, void* stream) {
+void launch_expand_state(bool h_half, const HalfStepParams<T>& p, bool o_kept, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (h_half) expand_state_kernel<T, true><<<cell_grid(p), 128, 0, st>>>(p);
-  else expand_state_kernel<T, false><<<cell_grid(p), 128, 0, st>>>(p);
+  if (h_half) expand_state_kernel<T, true><<<cell_grid(p), 128, 0, st>>>(p, o_kept);
+  else expand_state_kernel<T, false><<<cell_grid(p), 128, 0, st>>>(p, o_kept);
+}
+
+// O of the CPML cells where it is the state into the array of T, free there (KeepArgs):
+// one thread per cell of the absorber's layers.
+template <typename T>
+__global__ void __launch_bounds__(256) keep_state_kernel(const __grid_constant__ KeepArgs<T> a, bool from_t) {
+  const KeepHalf<T>& h = a.half[blockIdx.y];
+  for (long long u = blockIdx.x * 256ll + threadIdx.x; u < a.first[6]; u += gridDim.x * 256ll) {
+    int b = 0;
+    while (u >= a.first[b + 1]) ++b;
+    const long long e = u - a.first[b];
+    int at[3];
+    if (e <= 0xffffffffll) {  // 32-bit division wherever the index fits
+      const unsigned r = unsigned(e) / unsigned(a.dims[b][0]);
+      at[0] = a.start[b][0] + int(unsigned(e) - r * unsigned(a.dims[b][0]));
+      at[2] = a.start[b][2] + int(r / unsigned(a.dims[b][1]));
+      at[1] = a.start[b][1] + int(r % unsigned(a.dims[b][1]));
+    } else {
+      const long long r = e / a.dims[b][0];
+      at[0] = a.start[b][0] + int(e % a.dims[b][0]);
+      at[2] = a.start[b][2] + int(r / a.dims[b][1]);
+      at[1] = a.start[b][1] + int(r % a.dims[b][1]);
+    }
+    const long long q = a.origin + at[2] * a.plane + at[1] * a.pitch + at[0];
+    if (!KH_IN(q, a.total, 2151)) continue;
+    if (h.tile_bits) {  // special cells keep their T
+      const long long w = ((long long)(at[2] >> 6) * a.n[1] + at[1]) * a.nxb + (at[0] >> 6);
+      if (((h.tile_bits[w] >> (at[2] & 63)) & 1ull) && (a.cell_class[q] & h.special)) continue;
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      if (at[c] < h.lo[c] || at[c] >= a.n[c] - h.hi[c]) continue;  // T is the state
+      const T o = h.O[c][q];
+      if (!from_t) {
+        h.Ts[c][q] = o;
+      } else {
+        const T mt = mul_rn(h.m_inv[c] ? h.m_inv[c][q] : h.m_scalar, h.Ts[c][q]);
+        h.Ts[c][q] = fabs(o - mt) <= derived_tol(mt) ? o : mt;
+      }
+    }
+  }
+}
+
+template <typename T>
+void launch_keep_state(const KeepArgs<T>& a, int halves, bool from_t, void* stream) {
+  if (a.first[6] <= 0) return;
+  const dim3 grid(unsigned(std::min<long long>((a.first[6] + 255) / 256, 1 << 30)), unsigned(halves));
+  keep_state_kernel<T><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(a, from_t);
 }
 
 // What the reduced state takes for granted, checked on the complete T, U and W of a
@@ -437,8 +543,6 @@ template <typename T, bool H>
 __global__ void check_state_kernel(const HalfStepParams<T> p, StateCheck<T>* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.nx) return;
-  const T eps = sizeof(T) == 4 ? T(1.1920929e-7) : T(2.220446049250313e-16);
-  const T tiny = sizeof(T) == 4 ? T(1.17549435e-38) : T(2.2250738585072014e-308);
   bool broken = false;
   T top_t = T(0), off_u = T(0), top_o = T(0), off_o = T(0);
   // the largest so far; NaN counts as infinite
@@ -447,9 +551,8 @@ __global__ void check_state_kernel(const HalfStepParams<T> p, StateCheck<T>* out
   };
   for (int k = blockIdx.z; k < p.nz; k += gridDim.z)
     for (int j = blockIdx.y; j < p.ny; j += gridDim.y) {
-      const bool f[3] = {i < p.pml_lo[0] || i >= p.nx - p.pml_hi[0], j < p.pml_lo[1] || j >= p.ny - p.pml_hi[1],
-                         k < p.pml_lo[2] || k >= p.nz - p.pml_hi[2]};
-      if (!(f[0] || f[1] || f[2])) continue;
+      bool f[3];
+      if (!in_absorber(p, i, j, k, f)) continue;
       const long long q = p.origin + (long long)k * p.plane + (long long)j * p.pitch + i;
       if (!KH_IN(q, p.total, 2150)) continue;
       if (p.cell_class && (p.cell_class[q] & (H ? kSpecialH : kSpecialE))) continue;  // keeps the complete state
@@ -459,7 +562,7 @@ __global__ void check_state_kernel(const HalfStepParams<T> p, StateCheck<T>* out
         const int n = (c + 1) % 3, v = (c + 2) % 3;
         const T t = p.Ts[c][q], o = p.O[c][q];
         const T mt = mul_rn(p.m_inv[c] ? p.m_inv[c][q] : p.m_scalar, t);
-        const T near = T(8) * (eps * fabs(mt) + tiny);
+        const T near = derived_tol(mt);
         if (f[c] && p.ax[c][idx[c]].s != T(0)) {
           broken |= !(fabs(p.W[c][q] - mt) <= near);
         } else if (!f[c]) {
@@ -492,6 +595,19 @@ void launch_check_state(bool h_half, const HalfStepParams<T>& p, StateCheck<T>* 
   else check_state_kernel<T, false><<<cell_grid(p), 128, 0, st>>>(p, out);
 }
 
+// VIEW forms: the second where the first spills.
+template <typename T, bool PV>
+constexpr int view_forms() {
+  return sizeof(T) == 4 && PV ? 2 : 1;
+}
+
+template <typename T, bool H, bool PV, int VIEW>
+static void launch_view(dim3 grid, dim3 block, const HalfStepParams<T>& p, const TmaMaps& maps, cudaStream_t st) {
+  constexpr size_t smem = LeanGeom<T, PV>::SMEM;
+  if (p.wrap) half_step_lean_kernel<T, H, PV, false, true, VIEW><<<grid, block, smem, st>>>(p, maps);
+  else half_step_lean_kernel<T, H, PV, false, false, VIEW><<<grid, block, smem, st>>>(p, maps);
+}
+
 template <typename T, bool H, bool PV>
 static void launch_lean_variant(const HalfStepParams<T>& p, const TmaMaps& maps, cudaStream_t st) {
   const dim3 block(kLeanThreads, 1, 1);
@@ -501,6 +617,16 @@ static void launch_lean_variant(const HalfStepParams<T>& p, const TmaMaps& maps,
       half_step_lean_kernel<T, H, PV, true><<<grid, block, LeanGeom<T, PV>::SMEM, st>>>(p, maps);
       return;
     }
+  }
+  if (p.view) {
+    if constexpr (view_forms<T, PV>() == 2) {
+      if (p.view_form == 2) {
+        launch_view<T, H, PV, 2>(grid, block, p, maps, st);
+        return;
+      }
+    }
+    launch_view<T, H, PV, 1>(grid, block, p, maps, st);
+    return;
   }
   if (p.wrap) half_step_lean_kernel<T, H, PV, false, true><<<grid, block, LeanGeom<T, PV>::SMEM, st>>>(p, maps);
   else half_step_lean_kernel<T, H, PV><<<grid, block, LeanGeom<T, PV>::SMEM, st>>>(p, maps);
@@ -519,10 +645,16 @@ void launch_half_step_lean(bool h_half, const HalfStepParams<T>& p, const TmaMap
   }
 }
 
-template <typename T, bool H, bool PV, bool STALL = false, bool PER = false>
+template <typename T, bool H, bool PV, bool STALL = false, bool PER = false, int VIEW = 0>
 static int set_lean_attr() {
-  return int(cudaFuncSetAttribute(half_step_lean_kernel<T, H, PV, STALL, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return int(cudaFuncSetAttribute(half_step_lean_kernel<T, H, PV, STALL, PER, VIEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   int(LeanGeom<T, PV>::SMEM)));
+}
+
+template <typename T, bool PV, int VIEW>
+static int set_view_attr() {
+  return set_lean_attr<T, true, PV, false, false, VIEW>() | set_lean_attr<T, true, PV, false, true, VIEW>() |
+         set_lean_attr<T, false, PV, false, false, VIEW>() | set_lean_attr<T, false, PV, false, true, VIEW>();
 }
 
 template <typename T>
@@ -536,7 +668,9 @@ int prepare_lean_kernels() {
   e |= set_lean_attr<T, true, false, false, true>();
   e |= set_lean_attr<T, false, true, false, true>();
   e |= set_lean_attr<T, false, false, false, true>();
+  e |= set_view_attr<T, true, 1>() | set_view_attr<T, false, 1>();
   if constexpr (sizeof(T) == 4) {
+    e |= set_view_attr<T, true, 2>();
     e |= set_lean_attr<T, true, true, true>();
     e |= set_lean_attr<T, true, false, true>();
     e |= set_lean_attr<T, false, true, true>();
@@ -546,23 +680,27 @@ int prepare_lean_kernels() {
 }
 
 template <typename T>
-int lean_resident_ctas() {
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, half_step_lean_kernel<T, false, true>, kLeanThreads,
-                                                    LeanGeom<T, true>::SMEM) != cudaSuccess)
-    return 1;
-  return n > 0 ? n : 1;
+int lean_resident_ctas(int view) {
+  auto resident = [](auto kernel) {
+    int n = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kLeanThreads, LeanGeom<T, true>::SMEM);
+    return e == cudaSuccess && n > 0 ? n : 1;
+  };
+  if (view == 2 && sizeof(T) == 4) return resident(half_step_lean_kernel<T, false, true, false, false, sizeof(T) == 4 ? 2 : 1>);
+  return view ? resident(half_step_lean_kernel<T, false, true, false, false, 1>) : resident(half_step_lean_kernel<T, false, true>);
 }
 
 template void launch_half_step_lean<float>(bool, const HalfStepParams<float>&, const TmaMaps&, void*);
 template void launch_half_step_lean<double>(bool, const HalfStepParams<double>&, const TmaMaps&, void*);
-template void launch_expand_state<float>(bool, const HalfStepParams<float>&, void*);
-template void launch_expand_state<double>(bool, const HalfStepParams<double>&, void*);
+template void launch_expand_state<float>(bool, const HalfStepParams<float>&, bool, void*);
+template void launch_expand_state<double>(bool, const HalfStepParams<double>&, bool, void*);
+template void launch_keep_state<float>(const KeepArgs<float>&, int, bool, void*);
+template void launch_keep_state<double>(const KeepArgs<double>&, int, bool, void*);
 template void launch_check_state<float>(bool, const HalfStepParams<float>&, StateCheck<float>*, void*);
 template void launch_check_state<double>(bool, const HalfStepParams<double>&, StateCheck<double>*, void*);
 template int prepare_lean_kernels<float>();
 template int prepare_lean_kernels<double>();
-template int lean_resident_ctas<float>();
-template int lean_resident_ctas<double>();
+template int lean_resident_ctas<float>(int);
+template int lean_resident_ctas<double>(int);
 
 }  // namespace kh

@@ -39,6 +39,19 @@ __device__ __forceinline__ T curl_rn(T ca, T a1, T a0, T cb, T b1, T b0) {
   return fma_rn(ca, sub_rn(a1, a0), -mul_rn(cb, sub_rn(b1, b0)));
 }
 
+// T as it follows from O outside the own-axis CPML, and how far O may be from m·T (o)
+// by the rounding of both.
+template <typename T>
+__device__ __forceinline__ T derived_t(T O, T m) {
+  return m != T(0) ? O / m : T(0);
+}
+template <typename T>
+__device__ __forceinline__ T derived_tol(T o) {
+  constexpr T eps = sizeof(T) == 4 ? T(1.1920929e-7) : T(2.220446049250313e-16);
+  constexpr T tiny = sizeof(T) == 4 ? T(1.17549435e-38) : T(2.2250738585072014e-308);
+  return T(8) * (eps * fabs(o) + tiny);
+}
+
 // CPML factors of a cell along one axis; f false: outside that axis's CPML.
 template <typename T>
 struct RedAxis {

@@ -419,6 +419,16 @@ class Sim : public SimBase {
       lo_[a] = d_.pml_lo[a];
       hi_[a] = d_.pml_hi[a];
       pml_axis_[a] = lo_[a] > 0 || hi_[a] > 0;
+      for (int h = 0; h < 2; ++h) {
+        const std::vector<T>& sg = h ? sigb_h_[a] : sigd_h_[a];
+        int lo = lo_[a], hi = hi_[a];
+        while (lo > 0 && sg[lo - 1] == T(0)) --lo;
+        while (hi > 0 && sg[n_[a] - hi] == T(0)) --hi;
+        red_lo_[h][a] = lo;
+        red_hi_[h][a] = hi;
+        for (int i = 0; i < n_[a]; ++i)
+          if ((i < lo || i >= n_[a] - hi) && sg[i] == T(0)) sigma_gap_ = true;
+      }
     }
     const bool any_pml = pml_axis_[0] || pml_axis_[1] || pml_axis_[2];
 
@@ -857,7 +867,7 @@ class Sim : public SimBase {
     while (done < nsteps) {
       const int64_t to_edge = batch_len_ - timestep_ % batch_len_;
       const int nb = int(std::min<int64_t>(to_edge, nsteps - done));
-      kh_status st = run_batch(nb, stream);
+      kh_status st = run_batch(nb, stream, done == 0, done + nb == nsteps);
       if (st != KH_OK) return st;
       done += nb;
     }
@@ -1058,7 +1068,7 @@ class Sim : public SimBase {
       bool cpml = false;
       for (int a = 0; a < 3; ++a) cpml = cpml || st[a] < lo_[a] || st[a] + dm[a] > n_[a] - hi_[a];
       if (cpml) {
-        if (kh_status es = expand_state(); es != KH_OK) return es;
+        if (kh_status es = expand_state(half); es != KH_OK) return es;
         complete_[half] = kOneStep;
       }
     }
@@ -1156,6 +1166,15 @@ class Sim : public SimBase {
   kh_status field_view(int comp, kh_field_view* out) override {
     if (!prepared_) return fail(KH_ERR_INVALID, "field view before prepare");
     if (comp < 0 || comp > 5 || !out) return fail(KH_ERR_INVALID, "bad field view arguments");
+    if (const int h = comp < 3 ? 0 : 1; !views_out_[h]) {
+      // from here on the state of CPML cells is told from what is written there
+      if (kh_status es = wait_idle(); es != KH_OK) return es;
+      if (sigma_gap_)
+        if (kh_status es = expand_state(h); es != KH_OK) return es;
+      views_out_[h] = true;
+      stay_complete();
+      if (kh_status es = keep_state(1 << h, false); es != KH_OK) return es;
+    }
     T* base = comp < 3 ? E_[comp] : H_[comp - 3];
     out->data = base + origin_;
     out->dtype = dtype();
@@ -1185,6 +1204,7 @@ class Sim : public SimBase {
     timestep_ = 0;
     sources_active_ = true;
     complete_[0] = complete_[1] = kDerived;
+    stay_complete();
     return KH_OK;
   }
 
@@ -1197,7 +1217,8 @@ class Sim : public SimBase {
   kh_status export_state(void* dst, int64_t bytes) override {
     if (!prepared_ || !dst || bytes != state_bytes()) return fail(KH_ERR_INVALID, "bad export buffer");
     if (kh_status es = wait_idle(); es != KH_OK) return es;
-    if (kh_status es = expand_state(); es != KH_OK) return es;
+    for (int h = 0; h < 2; ++h)
+      if (kh_status es = expand_state(h); es != KH_OK) return es;
     char* p = static_cast<char*>(dst);
     int64_t hdr[2] = {timestep_, sources_active_ ? 1 : 0};
     std::memcpy(p, hdr, 16);
@@ -1206,7 +1227,7 @@ class Sim : public SimBase {
       KH_CUDA(cudaMemcpy(p, s.first, s.second, cudaMemcpyDeviceToHost));
       p += s.second;
     }
-    return KH_OK;
+    return keep_state(3, true);
   }
 
   kh_status import_state(const void* src, int64_t bytes) override {
@@ -1299,7 +1320,7 @@ class Sim : public SimBase {
     int64_t done = 0;
     while (done < nsteps) {
       const int nb = int(std::min<int64_t>(kBatch, nsteps - done));
-      kh_status st = run_batch(nb, stream, &t);
+      kh_status st = run_batch(nb, stream, done == 0, done + nb == nsteps, &t);
       if (st != KH_OK) return st;
       done += nb;
     }
@@ -1505,7 +1526,8 @@ class Sim : public SimBase {
     return s.table[q];
   }
 
-  kh_status run_batch(int nb, cudaStream_t stream, Timing* timing = nullptr) {
+  // nb steps; first, last: of the caller's steps.
+  kh_status run_batch(int nb, cudaStream_t stream, bool first, bool last, Timing* timing = nullptr) {
     // A batch on a new stream waits for the previous batch, whose kernels read
     // the shared time-factor table this batch is about to overwrite.
     if (last_stream_ != stream && batch_done_) KH_CUDA(cudaStreamWaitEvent(stream, batch_done_, 0));
@@ -1637,6 +1659,13 @@ class Sim : public SimBase {
       }
     };
     const bool whole = fused_ && !timing;
+    // views of the fields are out: O of CPML cells from its copy in a half's first step of
+    // the call, the copy from O in the last one (not where T is kept)
+    const bool any_cpml = pml_axis_[0] || pml_axis_[1] || pml_axis_[2];
+    auto view = [&](int h, int s) {
+      if (!views_out_[h] || !any_cpml) return 0u;
+      return (first && s == 0 ? kh::kViewRestore : 0u) | (last && s == nb - 1 ? kh::kViewKeep : 0u);
+    };
     auto issue_all = [&](cudaStream_t st) {
     for (int s = 0; s < nb; ++s) {
       // two whole steps, into the second set and back
@@ -1662,7 +1691,8 @@ class Sim : public SimBase {
       const bool src_h = P.sa && has_src_[1];
       ph.full = (full_h_base || (src_h && !src_lean_ok_[1]) || complete(1, s)) ? 1 : 0;
       mark(s, 0);
-      ph.zplanes = reduced_[1] && !ph.full ? zplanes_ : general_zplanes_;
+      ph.view = view(1, s);
+      ph.zplanes = reduced_[1] && !ph.full ? zplanes_[ph.view != 0] : general_zplanes_;
       if (reduced_[1] && !ph.full) kh::launch_half_step_lean<T>(true, ph, lean_maps_h_, st);
       else if (use_tma_) kh::launch_half_step_tma<T>(true, ph, maps_h_, st);
       else kh::launch_half_step<T>(true, ph, st);
@@ -1684,7 +1714,8 @@ class Sim : public SimBase {
       pe.f_now = dtab + P.fE;
       const bool src_e = P.sa && has_src_[0];
       pe.full = (full_e_base || (src_e && !src_lean_ok_[0]) || complete(0, s)) ? 1 : 0;
-      pe.zplanes = reduced_[0] && !pe.full ? zplanes_ : general_zplanes_;
+      pe.view = view(0, s);
+      pe.zplanes = reduced_[0] && !pe.full ? zplanes_[pe.view != 0] : general_zplanes_;
       if (reduced_[0] && !pe.full) kh::launch_half_step_lean<T>(false, pe, lean_maps_e_, st);
       else if (use_tma_) kh::launch_half_step_tma<T>(false, pe, maps_e_, st);
       else kh::launch_half_step<T>(false, pe, st);
@@ -1699,6 +1730,9 @@ class Sim : public SimBase {
       record_histories(false, timestep_ + s, st);
       mark(s, 4);
     }
+    // a call of one step through the complete state leaves T, and is back on the
+    // reduced one
+    if (last && nb == 1) launch_keep((complete_[0] == kOneStep ? 1 : 0) | (complete_[1] == kOneStep ? 2 : 0), true, st);
     };
     if (!use_graph) {
       issue_all(stream);
@@ -1709,7 +1743,8 @@ class Sim : public SimBase {
       sig.reserve(size_t(nb) * 8 + 4);
       sig.push_back(nb);
       sig.push_back(b);
-      sig.push_back(complete_[0] + 4 * complete_[1]);
+      sig.push_back(complete_[0] + 4 * complete_[1] + 16 * int(view(0, 0) | view(0, nb - 1)) +
+                    64 * int(view(1, 0) | view(1, nb - 1)));
       for (int q = 0; q < nb; ++q) {
         const StepPlan& P = plan[q];
         sig.push_back(P.sa ? 1 : 0);
@@ -1960,7 +1995,7 @@ class Sim : public SimBase {
     }
     KH_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
     if (sizeof(T) == 4) fused_slots_ = sms_ * kh::fused_resident_ctas<float>();
-    lean_slots_ = sms_ * kh::lean_resident_ctas<T>();
+    for (int v = 0; v < 3; ++v) lean_slots_[v] = sms_ * kh::lean_resident_ctas<T>(v);
     tma_slots_ = sms_ * kh::tma_resident_ctas<T>();
     const int hx = 16 / int(sizeof(T));
     struct MapSet {
@@ -1995,16 +2030,26 @@ class Sim : public SimBase {
 
   // z planes per CTA of the reduced-state and of the general half-step kernel.
   void choose_zplanes() {
-    zplanes_ = general_zplanes_ = std::min(10, n_[2]);
+    zplanes_[0] = zplanes_[1] = general_zplanes_ = std::min(10, n_[2]);
     if (use_tma_) {
-      zplanes_ = kh::reduced_zplanes(n_[2], kh::plan_tiles(n_[0], n_[1], kh::kLeanX, kh::kLeanY), lean_slots_, sms_,
-                                     sizeof(T) == 8, pml_axis_[0] || pml_axis_[1] || pml_axis_[2]);
+      const long long tiles = kh::plan_tiles(n_[0], n_[1], kh::kLeanX, kh::kLeanY);
+      auto depth = [&](int slots) {
+        return kh::reduced_zplanes(n_[2], tiles, slots, sms_, sizeof(T) == 8,
+                                   pml_axis_[0] || pml_axis_[1] || pml_axis_[2]);
+      };
+      zplanes_[0] = depth(lean_slots_[0]);
+      zplanes_[1] = depth(lean_slots_[1]);
+      const long long ctas = tiles * ((n_[2] + zplanes_[1] - 1) / zplanes_[1]);
+      if (ctas > lean_slots_[1] + lean_slots_[1] / 16) {
+        view_form_ = 2;
+        zplanes_[1] = depth(lean_slots_[2]);
+      }
       general_zplanes_ = kh::general_zplanes(n_[2], kh::plan_tiles(n_[0], n_[1], kh::kTmaX, kh::kTmaY), tma_slots_);
     }
     if (const char* zv = std::getenv("KHRONOS_GB300_ZPLANES")) {
       const int z = std::atoi(zv);
       if (z >= 1) {
-        zplanes_ = std::min({z, n_[2], kh::kLeanZ});
+        zplanes_[0] = zplanes_[1] = std::min({z, n_[2], kh::kLeanZ});
         general_zplanes_ = std::min(z, n_[2]);
       }
     }
@@ -2135,20 +2180,94 @@ class Sim : public SimBase {
       if (!(c[h].off_u <= drift * c[h].top_t)) complete_[h] = kStays;
       else if (c[h].broken || !(c[h].off_o <= drift * c[h].top_o)) complete_[h] = kOneStep;
     }
-    return KH_OK;
+    stay_complete();
+    return keep_state(3, true);
   }
 
-  // T, U and W of every CPML cell brought up to date from the reduced state.
-  kh_status expand_state() {
-    if (!(pml_axis_[0] || pml_axis_[1] || pml_axis_[2])) return KH_OK;
-    for (int h = 0; h < 2; ++h) {
-      if (!reduced_[h] || complete_[h] != kDerived) continue;
-      kh::launch_expand_state<T>(h == 1, base_params(h == 1), cudaStreamLegacy);
-      ++launches;
-    }
+  // Where σ = 0 between layers that damp, the reduced state sums O up beside T, and a
+  // value written through a view would stay: such a program's steps keep all of it.
+  void stay_complete() {
+    for (int h = 0; h < 2; ++h)
+      if (views_out_[h] && sigma_gap_ && reduced_[h]) complete_[h] = kStays;
+  }
+
+  bool reduced_cpml(int h) const {
+    return reduced_[h] && complete_[h] == kDerived && (pml_axis_[0] || pml_axis_[1] || pml_axis_[2]);
+  }
+
+  // T, U and W of every CPML cell of a half brought up to date from the reduced state.
+  kh_status expand_state(int h) {
+    if (!reduced_cpml(h)) return KH_OK;
+    kh::launch_expand_state<T>(h == 1, base_params(h == 1), views_out_[h], cudaStreamLegacy);
+    ++launches;
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e != cudaSuccess) return fail(KH_ERR_CUDA, std::string("state expansion: ") + cudaGetErrorString(e));
+    return KH_OK;
+  }
+
+  // The copies of the halves in mask (bit 0: E, bit 1: H) that views are out of.
+  void launch_keep(int mask, bool from_t, cudaStream_t st) {
+    if (!(pml_axis_[0] || pml_axis_[1] || pml_axis_[2])) return;
+    kh::KeepArgs<T> a;
+    std::memset(&a, 0, sizeof(a));
+    int halves = 0;
+    for (int h = 0; h < 2; ++h) {
+      if (!((mask >> h) & 1) || !reduced_[h] || !views_out_[h]) continue;
+      kh::KeepHalf<T>& k = a.half[halves++];
+      for (int c = 0; c < 3; ++c) {
+        k.O[c] = h ? H_[c] : E_[c];
+        k.Ts[c] = h ? B_[c] : D_[c];
+        k.m_inv[c] = h ? mu_[c] : eps_[c];
+        k.lo[c] = red_lo_[h][c];
+        k.hi[c] = red_hi_[h][c];
+      }
+      k.m_scalar = h ? T(d_.mu_inv) : T(d_.eps_inv);
+      k.tile_bits = h ? tbits_h_ : tbits_e_;
+      k.special = h ? kh::kSpecialH : kh::kSpecialE;
+    }
+    if (!halves) return;
+    a.nxb = nxb_;
+    a.pitch = pitch_;
+    a.plane = plane_;
+    a.origin = origin_;
+    a.total = total_;
+    a.cell_class = cls_;
+    // whole z layers, then y layers between them, then x layers between those
+    int from[3], to[3];
+    for (int c = 0; c < 3; ++c) {
+      a.n[c] = n_[c];
+      from[c] = 0;
+      to[c] = n_[c];
+    }
+    for (int b = 0; b < 6; ++b) {
+      const int ax = 2 - b / 2;
+      for (int c = 0; c < 3; ++c) {
+        a.start[b][c] = from[c];
+        a.dims[b][c] = to[c] - from[c];
+      }
+      if (b % 2 == 0) {
+        a.dims[b][ax] = lo_[ax];
+        from[ax] = lo_[ax];
+      } else {
+        a.start[b][ax] = n_[ax] - hi_[ax];
+        a.dims[b][ax] = hi_[ax];
+        to[ax] = n_[ax] - hi_[ax];
+      }
+      a.first[b + 1] = a.first[b] + 1ll * a.dims[b][0] * a.dims[b][1] * a.dims[b][2];
+    }
+    kh::launch_keep_state<T>(a, halves, from_t, st);
+    ++launches;
+  }
+
+  // The copies that the next call starts from (from_t: out of the complete state).
+  kh_status keep_state(int mask, bool from_t) {
+    if (!views_out_[0] && !views_out_[1]) return KH_OK;
+    launch_keep(mask & ((complete_[0] == kDerived ? 1 : 0) | (complete_[1] == kDerived ? 2 : 0)), from_t,
+                cudaStreamLegacy);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    if (e != cudaSuccess) return fail(KH_ERR_CUDA, std::string("state copy: ") + cudaGetErrorString(e));
     return KH_OK;
   }
 
@@ -2281,7 +2400,10 @@ class Sim : public SimBase {
       p.ax[c] = h ? axb_[c] : axd_[c];
       p.pml_lo[c] = lo_[c];
       p.pml_hi[c] = hi_[c];
+      p.red_lo[c] = red_lo_[h][c];
+      p.red_hi[c] = red_hi_[h][c];
     }
+    p.view_form = view_form_;
     p.cpml = d_.semantics == KH_SEM_CPML ? 1 : 0;
     p.m_scalar = h ? T(d_.mu_inv) : T(d_.eps_inv);
     p.sigma_region_mask = h ? sigmask_b_ : sigmask_d_;
@@ -2326,6 +2448,8 @@ class Sim : public SimBase {
   int nxb_;
   int lo_[3] = {0, 0, 0}, hi_[3] = {0, 0, 0};
   bool pml_axis_[3] = {false, false, false};
+  int red_lo_[2][3] = {}, red_hi_[2][3] = {};  // [E half, H half]: HalfStepParams::red_lo, red_hi
+  bool sigma_gap_ = false;  // σ = 0 inside those, too
   uint32_t sigmask_b_ = 0, sigmask_d_ = 0;
   bool prepared_ = false;
 
@@ -2370,12 +2494,13 @@ class Sim : public SimBase {
   bool disp_fix_ = false;      // χ3 / pole cells by the dispersive-cell pass after a LEAN E launch
   uint32_t* disp_list_ = nullptr;  // its row-segment list (DispFixParams::list)
   int n_disp_list_ = 0;
-  int zplanes_ = 10, general_zplanes_ = 10;  // of kh_lean.cu, of kh_tma.cu
+  int zplanes_[2] = {10, 10}, general_zplanes_ = 10;  // of kh_lean.cu (and its VIEW forms), of kh_tma.cu
+  int view_form_ = 1;
   int xprefetch_ = 2;        // x-CPML state prefetch mode (HalfStepParams::xprefetch)
   int xpf_dist_ = 3;
   int sms_ = 1;
   int fused_slots_ = 1;  // SMs × resident whole-step CTAs per SM
-  int lean_slots_ = 1, tma_slots_ = 1;  // … reduced-state, general-kernel CTAs per SM
+  int lean_slots_[3] = {1, 1, 1}, tma_slots_ = 1;  // … reduced-state, general-kernel CTAs per SM
   kh::TmaMaps maps_h_, maps_e_;            // kTmaY rows (general kernel)
   kh::TmaMaps lean_maps_h_, lean_maps_e_;  // kLeanY rows (reduced-state kernel)
   // [E half, H half]: the reduced-state kernel takes this half's launches.  T, U
@@ -2387,6 +2512,9 @@ class Sim : public SimBase {
   // imported state is another absorber's).
   enum { kDerived = 0, kOneStep = 1, kStays = 2 };
   int complete_[2] = {kDerived, kDerived};
+  // [E, H]: kh_sim_field_view was called: between calls the arrays of T hold a copy of O
+  // in CPML cells where O is the state (where complete_ is kDerived)
+  bool views_out_[2] = {false, false};
   // Whole-step launches (kh_fused.cu): the second set of E and H, the tensor maps
   // from set 0 into 1 and back, and the set that holds the current fields (1 only
   // between the two steps of a pair).

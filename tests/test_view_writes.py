@@ -1,0 +1,130 @@
+"""Writes through field views: what the header says of them.  They change the simulation;
+values at cells that keep B/D state are recomputed from that state at the next step.
+In the absorber the reduced state keeps no D where E stands for it, so the first step of
+a call has to tell a written value from the state.  Against the register-pipelined kernel, which
+keeps the complete state (same recurrences up to rounding)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"f32": 2e-4, "f64": 1e-10}
+
+
+def _spec(kh, dtype, n, pml, voxel=True, sources=True):
+    srcs = [kh.UniformSource(time_profile=kh.GaussianPulseSource(fcen=0.8, fwidth=0.6), component=c,
+                             center=(0.1, 0.05, 0), size=(0, 0.9 * n[1] / 10, 0.6)) for c in (kh.EY, kh.HX)]
+    sp = kh.Simulation(cell_size=tuple(a / 10 for a in n), resolution=10, sources=srcs if sources else [],
+                       boundaries=[[w / 10, w / 10] for w in pml], dtype=dtype).spec()
+    assert tuple(sp.n) == n
+    rng = np.random.default_rng(3)
+    if voxel:
+        for kind in (0, 1):
+            for c in range(3):  # values exact in single precision
+                sp.materials.append((kind, c, rng.integers(16, 32, size=n) / 32.0))
+    return sp
+
+
+def _same(a, b, tol):
+    fa, fb = [a.field(c) for c in range(6)], [b.field(c) for c in range(6)]
+    for grp in ((0, 1, 2), (3, 4, 5)):
+        scale = np.sqrt(sum(np.sum(fb[c] ** 2) for c in grp))
+        assert scale > 0
+        for c in grp:
+            assert np.linalg.norm(fa[c] - fb[c]) <= tol * scale, c
+
+
+def _write(g, seed, n, scale):
+    import torch
+
+    rng = np.random.default_rng(seed)
+    g.synchronize()
+    for c in range(6):
+        v = g.field_view(c)
+        add = torch.as_tensor(rng.integers(-32, 32, size=n) / 32.0 * scale, device=v.device, dtype=v.dtype)
+        v[:n[0], :n[1], :n[2]].mul_(0.5).add_(add)  # the cells that are updated, not the wall layer
+    torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+@pytest.mark.parametrize("n,pml,voxel", [((70, 22, 18), (5, 4, 3), True), ((70, 22, 18), (5, 4, 3), False),
+                                         ((61, 9, 14), (6, 0, 0), True), ((40, 14, 20), (0, 4, 5), False),
+                                         ((200, 100, 60), (5, 4, 3), True)])  # more than one round of CTAs
+def test_writes_in_mid_run(kh, gpu_lib, monkeypatch, dtype, n, pml, voxel):
+    from khronos_gb300.device import GpuSim
+
+    sp = _spec(kh, dtype, n, pml, voxel)
+    a = GpuSim(sp, lib=gpu_lib)
+    monkeypatch.setenv("KHRONOS_GB300_KERNEL", "simt")
+    b = GpuSim(sp, lib=gpu_lib)
+    for g in (a, b):
+        g.step(25)
+        _write(g, 1, n, 2.0 ** -6)
+        g.step(1)
+        _write(g, 2, n, 2.0 ** -6)
+        g.step(9)
+    _same(a, b, TOL[dtype])
+    for g in (a, b):  # a written state exported, and gone on from as it is
+        _write(g, 3, n, 2.0 ** -6)
+        g.export_state()
+        g.step(7)
+        if voxel:
+            _write(g, 4, n, 2.0 ** -6)
+            g.update_material_box(0, 1, (0, 0, 0), np.full((n[0], 3, n[2]), 0.75))
+        g.step(1)
+        _write(g, 5, n, 2.0 ** -6)
+        g.step(4)
+        g.step_timed(6)
+    _same(a, b, TOL[dtype])
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+@pytest.mark.parametrize("gap", [False, True])
+def test_initial_fields(kh, gpu_lib, monkeypatch, dtype, gap):
+    from khronos_gb300.device import GpuSim
+
+    n = (70, 22, 18)
+    sp = _spec(kh, dtype, n, (5, 4, 3), sources=False)
+    if gap:  # an undamped layer between damped ones
+        for sg in (sp.sigma_b, sp.sigma_d):
+            for a in range(3):
+                sg[a] = np.array(sg[a])
+                sg[a][1] = sg[a][n[a] - 2] = 0.0
+    a = GpuSim(sp, lib=gpu_lib)
+    monkeypatch.setenv("KHRONOS_GB300_KERNEL", "simt")
+    b = GpuSim(sp, lib=gpu_lib)
+    for g in (a, b):
+        _write(g, 1, n, 1.0)
+        g.step(30)
+    _same(a, b, TOL[dtype])
+    for g in (a, b):
+        g.reset()
+        _write(g, 2, n, 1.0)
+        g.step(12)
+    _same(a, b, TOL[dtype])
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+@pytest.mark.parametrize("periodic", [0, 6])
+def test_views_that_are_only_read_change_no_bits(kh, gpu_lib, dtype, periodic):
+    from khronos_gb300.device import GpuSim
+
+    n = (70, 22, 18)
+    sp = _spec(kh, dtype, n, (5, 0, 0) if periodic else (5, 4, 3))
+    sp.periodic = periodic
+    a, b = GpuSim(sp, lib=gpu_lib), GpuSim(sp, lib=gpu_lib)
+    views = [a.field_view(c) for c in range(6)]
+    for steps in (1, 30, 2, 1, 150):
+        a.step(steps)
+        b.step(steps)
+        a.synchronize()
+        for c in range(6):
+            assert np.array_equal(a.field(c), b.field(c)), (steps, c)
+            assert np.array_equal(views[c].double().cpu().numpy(), a.field(c))
+    del views
+    a.close()
+    b.close()
