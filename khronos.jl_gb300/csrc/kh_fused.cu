@@ -25,6 +25,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "../../include/khronos_gb300.h"
 #include "kh_async.cuh"
 #include "kh_lean.cuh"
@@ -104,7 +106,7 @@ __global__ void __launch_bounds__(32 * kFusedRows, PV ? kFusedMinBlocks : kFused
         tma_load_3d(dst + 3 * (G::E_ELEMS + G::H_ELEMS) + c * G::M_ELEMS, &maps.m[c], px, y_own + 1, zc, &bars[st]);
     }
   };
-  const int l0 = k0 == 0 ? 1 : 0;  // the plane below the grid is zero
+  const int l0 = k0 == 0 ? 1 : 0;  // nothing is updated below the grid
   if (issuer)
     for (int l = l0; l < min(l0 + kFusedStages, N + 2); ++l) issue(l, l - l0);
 
@@ -133,6 +135,13 @@ __global__ void __launch_bounds__(32 * kFusedRows, PV ? kFusedMinBlocks : kFused
   const int ea = wy * G::EX + lane * VN;  // this thread's cells in the E box
   const int ha = wy * kTmaX + lane * VN;  // … in the H box
   PK hz0{}, hz1{};                        // new H0, H1 of the plane below
+  if (own && k0 == 0) {                   // … the ring below the grid
+    const long long qb = q - p.plane;
+    if (KH_IN(qb, p.total, 2204) && KH_IN(qb + VN - 1, p.total, 2204)) {
+      hz0 = *reinterpret_cast<const PK*>(p.Ho[0] + qb);
+      hz1 = *reinterpret_cast<const PK*>(p.Ho[1] + qb);
+    }
+  }
   int gave_up = -1;
   int st = 0;
   uint32_t parity = 0;
@@ -260,6 +269,44 @@ __global__ void __launch_bounds__(32 * kFusedRows, PV ? kFusedMinBlocks : kFused
                       kSleepWaitLimit);
 }
 
+// The ring around the grid (ghost and wall layers) from one set into the other, one
+// thread per element: the two x faces with their edges, the y faces with theirs along
+// z, the z faces.
+template <typename T>
+__global__ void __launch_bounds__(256) mirror_ring_kernel(const RingArgs<T> a) {
+  const T* from = a.from[blockIdx.y];
+  T* to = a.to[blockIdx.y];
+  const long long fx = 2ll * (a.ny + 2) * (a.nz + 2), fy = 2ll * a.nx * (a.nz + 2), fz = 2ll * a.nx * a.ny;
+  for (long long u = blockIdx.x * 256ll + threadIdx.x; u < fx + fy + fz; u += gridDim.x * 256ll) {
+    int x, y, z;
+    if (u < fx) {
+      const long long e = u >> 1;
+      x = u & 1 ? a.nx : -1;
+      y = int(e % (a.ny + 2)) - 1;
+      z = int(e / (a.ny + 2)) - 1;
+    } else if (u < fx + fy) {
+      const long long e = u - fx, r = e / a.nx;
+      x = int(e % a.nx);
+      y = r & 1 ? a.ny : -1;
+      z = int(r >> 1) - 1;
+    } else {
+      const long long e = u - fx - fy, r = e / a.nx;
+      x = int(e % a.nx);
+      y = int(r % a.ny);
+      z = r >= a.ny ? a.nz : -1;
+    }
+    const long long q = a.origin + z * a.plane + y * a.pitch + x;
+    if (KH_IN(q, a.total, 2250)) to[q] = from[q];
+  }
+}
+
+template <typename T>
+void launch_mirror_ring(const RingArgs<T>& a, void* stream) {
+  const long long n = 2ll * (a.ny + 2) * (a.nz + 2) + 2ll * a.nx * (a.nz + 2) + 2ll * a.nx * a.ny;
+  const dim3 grid(unsigned(std::min<long long>((n + 255) / 256, 1 << 20)), 6);
+  mirror_ring_kernel<T><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+}
+
 template <typename T>
 void launch_step_fused(const FusedParams<T>& p, const FusedMaps& maps, void* stream) {
   const dim3 block(32, kFusedRows, 1);
@@ -290,6 +337,7 @@ int fused_resident_ctas() {
 }
 
 template void launch_step_fused<float>(const FusedParams<float>&, const FusedMaps&, void*);
+template void launch_mirror_ring<float>(const RingArgs<float>&, void*);
 template int prepare_fused_kernels<float>();
 template int fused_resident_ctas<float>();
 

@@ -283,6 +283,7 @@ struct FusedParams {
   T cd[3];
   T mu_scalar, eps_scalar;
   T *En[3], *Hn[3];
+  const T* Ho[2];  // old H0, H1
   T* D[3];  // D state of special cells, in place
   const uint64_t* tile_bits;
   long long n_tile_words;
@@ -295,6 +296,18 @@ struct FusedParams {
 struct alignas(128) FusedMaps {
   CUtensorMap e[3], h[3], m[3];
 };
+
+// The six arrays whose ring (everything outside the grid) is copied from one set into
+// the other: it is never written by the kernels, but can be through a field view.
+template <typename T>
+struct RingArgs {
+  const T* from[6];
+  T* to[6];
+  int nx, ny, nz;
+  long long pitch, plane, origin, total;
+};
+template <typename T>
+void launch_mirror_ring(const RingArgs<T>& a, void* stream);
 
 template <typename T>
 void launch_step_fused(const FusedParams<T>& p, const FusedMaps& maps, void* stream);

@@ -1666,11 +1666,14 @@ class Sim : public SimBase {
       if (!views_out_[h] || !any_cpml) return 0u;
       return (first && s == 0 ? kh::kViewRestore : 0u) | (last && s == nb - 1 ? kh::kViewKeep : 0u);
     };
+    // … and what may have been written outside the grid goes into the second set, too
+    const bool mirror = first && (views_out_[0] || views_out_[1]);
     auto issue_all = [&](cudaStream_t st) {
     for (int s = 0; s < nb; ++s) {
       // two whole steps, into the second set and back
       if (whole && s + 1 < nb) {
         pe.full = 0;
+        if (mirror && s == 0) launch_mirror(st);
         for (int q = 0; q < 2; ++q) {
           const StepPlan& P = plan[s + q];
           launch_fused(q, st);
@@ -1744,7 +1747,7 @@ class Sim : public SimBase {
       sig.push_back(nb);
       sig.push_back(b);
       sig.push_back(complete_[0] + 4 * complete_[1] + 16 * int(view(0, 0) | view(0, nb - 1)) +
-                    64 * int(view(1, 0) | view(1, nb - 1)));
+                    64 * int(view(1, 0) | view(1, nb - 1)) + (whole && mirror ? 256 : 0));
       for (int q = 0; q < nb; ++q) {
         const StepPlan& P = plan[q];
         sig.push_back(P.sa ? 1 : 0);
@@ -2138,12 +2141,34 @@ class Sim : public SimBase {
         p.En[c] = from ? E_[c] : E2_[c];
         p.Hn[c] = from ? H_[c] : H2_[c];
         p.D[c] = D_[c];
+        if (c < 2) p.Ho[c] = from ? H2_[c] : H_[c];
       }
       p.tile_bits = tbits_e_;
       p.n_tile_words = tbits_e_ ? (long long)((n_[2] + 63) / 64) * n_[1] * nxb_ : 0;
       p.cell_class = cls_;
       p.err = err_dev_;
       kh::launch_step_fused<T>(p, fused_maps_[from], st);
+      ++launches;
+    }
+  }
+
+  void launch_mirror(cudaStream_t st) {
+    if constexpr (sizeof(T) == 4) {
+      kh::RingArgs<T> a;
+      for (int c = 0; c < 3; ++c) {
+        a.from[c] = E_[c];
+        a.to[c] = E2_[c];
+        a.from[3 + c] = H_[c];
+        a.to[3 + c] = H2_[c];
+      }
+      a.nx = n_[0];
+      a.ny = n_[1];
+      a.nz = n_[2];
+      a.pitch = pitch_;
+      a.plane = plane_;
+      a.origin = origin_;
+      a.total = total_;
+      kh::launch_mirror_ring<T>(a, st);
       ++launches;
     }
   }

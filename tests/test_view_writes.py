@@ -128,3 +128,40 @@ def test_views_that_are_only_read_change_no_bits(kh, gpu_lib, dtype, periodic):
     del views
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("n", [(61, 9, 14), (130, 15, 6)])
+def test_wall_layers_of_a_closed_box(kh, gpu_lib, monkeypatch, n):
+    """Values written into the staggered wall layers (and the ring below) act on every
+    step, whole steps through the second set of arrays as half-steps: the same bits."""
+    import torch
+
+    from khronos_gb300.device import GpuSim
+
+    sp = _spec(kh, "f32", n, (0, 0, 0))
+    sp.materials = [m for m in sp.materials if m[0] == 0]
+    sp.sources = [s for s in sp.sources if s.component < 3]
+    a = GpuSim(sp, lib=gpu_lib)
+    monkeypatch.setenv("KHRONOS_GB300_FUSED", "0")
+    b = GpuSim(sp, lib=gpu_lib)
+    rng = np.random.default_rng(8)
+    walls = [[rng.standard_normal((n[1] + 3, n[2] + 3, 2)), rng.standard_normal((n[0] + 3, n[2] + 3, 2)),
+              rng.standard_normal((n[0] + 3, n[1] + 3, 2))] for _ in range(6)]
+    for steps in (6, 7, 40):
+        for g in (a, b):
+            g.synchronize()
+            for c in range(6):
+                v = g.field_view(c, ghosted=True)  # layer -1 first, the staggered layer last
+                for ax in range(3):
+                    for side, at in enumerate((0, n[ax] + 1)):
+                        if at < v.shape[ax]:
+                            w = v.select(ax, at)
+                            w.copy_(torch.as_tensor(walls[c][ax][:w.shape[0], :w.shape[1], side] * 0.01,
+                                                    device=v.device, dtype=v.dtype))
+            torch.cuda.synchronize()
+            g.step(steps)
+        for c in range(6):
+            assert np.array_equal(a.field(c), b.field(c)), (steps, c)
+    assert a.launches < b.launches  # whole steps were taken
+    a.close()
+    b.close()
