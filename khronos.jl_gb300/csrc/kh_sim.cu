@@ -2076,12 +2076,15 @@ class Sim : public SimBase {
       size_t free_b = 0, all_b = 0;
       KH_CUDA(cudaMemGetInfo(&free_b, &all_b));
       if (6 * field > free_b / 16) return KH_OK;
-      for (int c = 0; c < 6; ++c)
-        if (alloc_raw(field, (void**)(c < 3 ? &E2_[c] : &H2_[c - 3]), false) != KH_OK) {
-          cudaGetLastError();  // somebody took the memory: half-steps
-          err.clear();
-          return KH_OK;
-        }
+      // one block for all six, or none: memory is then short, and half-steps do without
+      const size_t each = (field + 255) / 256 * 256;
+      char* second = nullptr;
+      if (alloc_raw(6 * each, (void**)&second, false) != KH_OK) {
+        cudaGetLastError();
+        err.clear();
+        return KH_OK;
+      }
+      for (int c = 0; c < 6; ++c) (c < 3 ? E2_[c] : H2_[c - 3]) = reinterpret_cast<T*>(second + size_t(c) * each);
       for (int h = 0; h < 2; ++h) {
         kh::FusedMaps& fm = fused_maps_[h];
         std::memset(&fm, 0, sizeof(fm));
