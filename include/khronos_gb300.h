@@ -426,8 +426,10 @@ kh_status kh_sim_import_state(kh_sim* sim, const void* host_src, int64_t bytes);
 /* Compulsory-traffic model of one full step (bytes): the reference's 9 + 12
  * words per cell (benchmark/benchmark_metrics.jl:236-241) plus CPML
  * auxiliaries, dispersive and χ3 terms, plus DFT monitor traffic amortised
- * over the decimation.  The split gives the H half-step kernel, the E
- * half-step kernel and the DFT launches separately. */
+ * over the decimation.  Where steps run as whole steps (FP32 grids without CPML,
+ * with the second set of E and H of kh_sim_memory_bytes) the fields count 12 words
+ * instead of 18.  The split gives the H half-step kernel, the E half-step kernel
+ * and the DFT launches separately, for steps in halves. */
 kh_status kh_sim_model_bytes_per_step(const kh_sim* sim, double* out);
 kh_status kh_sim_model_bytes_split(const kh_sim* sim, double* h_half, double* e_half,
                                    double* dft);
@@ -436,7 +438,9 @@ kh_status kh_sim_model_bytes_split(const kh_sim* sim, double* h_half, double* e_
  * (H half-step, E half-step, DFT) of every 8th step of the call (its first
  * step included); returns the device time (ms) of the H half-step kernels, the E
  * half-step kernels and the DFT launches of these nsteps, the sampled steps'
- * sums scaled to all nsteps.  No step-graph replay in timed runs. */
+ * sums scaled to all nsteps.  No step-graph replay in timed runs, and no whole
+ * steps: on grids where kh_sim_step takes those, these are the times of the two
+ * half-steps it would run without. */
 kh_status kh_sim_step_timed(kh_sim* sim, int64_t nsteps, void* stream, double* h_ms,
                             double* e_ms, double* dft_ms);
 
