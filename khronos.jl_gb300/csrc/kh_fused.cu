@@ -54,7 +54,7 @@ struct FusedGeom {
 
 }  // namespace
 
-template <typename T, bool PV>
+template <typename T, bool PV, bool STALL = false>
 __global__ void __launch_bounds__(32 * kFusedRows, PV ? kFusedMinBlocks : kFusedMinBlocks + 1)
     step_fused_kernel(const __grid_constant__ FusedParams<T> p, const __grid_constant__ FusedMaps maps) {
   using G = FusedGeom<T, PV>;
@@ -88,10 +88,18 @@ __global__ void __launch_bounds__(32 * kFusedRows, PV ? kFusedMinBlocks : kFused
   }
   __syncthreads();
 
+  constexpr int kLimit = STALL ? kStallSleepWaitLimit : kSleepWaitLimit;
+  const int l0 = k0 == 0 ? 1 : 0;  // nothing is updated below the grid
   // load l: plane k0 - 1 + l; the last one (plane k1) brings only what the H
   // update below it reads
   auto issue = [&](int l, int st) {
     T* dst = stages + st * G::STAGE;
+    if (STALL && l == l0) {
+      // failure-detection test instantiation: the first stage expects 16 bytes
+      // and no copy is issued into it, so the wait on it runs out
+      mbar_arrive_expect_tx(&bars[st], 16u);
+      return;
+    }
     const bool last = l == N + 1;
     mbar_arrive_expect_tx(&bars[st], (last ? 2u : 3u) * uint32_t(G::E_BYTES) +
                                          (last ? 0u : 3u * uint32_t(G::H_ELEMS * sizeof(T))) +
@@ -106,7 +114,6 @@ __global__ void __launch_bounds__(32 * kFusedRows, PV ? kFusedMinBlocks : kFused
         tma_load_3d(dst + 3 * (G::E_ELEMS + G::H_ELEMS) + c * G::M_ELEMS, &maps.m[c], px, y_own + 1, zc, &bars[st]);
     }
   };
-  const int l0 = k0 == 0 ? 1 : 0;  // nothing is updated below the grid
   if (issuer)
     for (int l = l0; l < min(l0 + kFusedStages, N + 2); ++l) issue(l, l - l0);
 
@@ -145,7 +152,7 @@ __global__ void __launch_bounds__(32 * kFusedRows, PV ? kFusedMinBlocks : kFused
   int gave_up = -1;
   int st = 0;
   uint32_t parity = 0;
-  if (!mbar_wait_sleep(smem_u32(bars), 0u, kSleepWaitLimit)) {
+  if (!mbar_wait_sleep(smem_u32(bars), 0u, kLimit)) {
     gave_up = l0;
     if (p.err) atomicExch(p.err, KH_ERR_TIMEOUT);
   }
@@ -162,7 +169,7 @@ __global__ void __launch_bounds__(32 * kFusedRows, PV ? kFusedMinBlocks : kFused
 #pragma unroll
       for (int c = 0; c < 3; ++c) D.c[c] = *reinterpret_cast<const PK*>(p.D[c] + q);
     }
-    if (gave_up < 0 && !mbar_wait_sleep(smem_u32(bars + sn), pn, kSleepWaitLimit)) {
+    if (gave_up < 0 && !mbar_wait_sleep(smem_u32(bars + sn), pn, kLimit)) {
       gave_up = l;
       if (p.err) atomicExch(p.err, KH_ERR_TIMEOUT);
     }
@@ -266,7 +273,7 @@ __global__ void __launch_bounds__(32 * kFusedRows, PV ? kFusedMinBlocks : kFused
   if (issuer && gave_up >= 0)
     for (int l = gave_up; l < min(gave_up + kFusedStages, N + 2); ++l)
       mbar_wait_sleep(smem_u32(bars + (l - l0) % kFusedStages), uint32_t(((l - l0) / kFusedStages) & 1),
-                      kSleepWaitLimit);
+                      kLimit);
 }
 
 // The ring around the grid (ghost and wall layers) from one set into the other, one
@@ -313,18 +320,25 @@ void launch_step_fused(const FusedParams<T>& p, const FusedMaps& maps, void* str
   const dim3 grid((p.nx + p.tile_w - 1) / p.tile_w, (p.ny + kFusedRows - 2) / (kFusedRows - 1),
                   (p.nz + p.zplanes - 1) / p.zplanes);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (p.stall_tx) {
+    if (p.pervox_eps) step_fused_kernel<T, true, true><<<grid, block, FusedGeom<T, true>::SMEM, st>>>(p, maps);
+    else step_fused_kernel<T, false, true><<<grid, block, FusedGeom<T, false>::SMEM, st>>>(p, maps);
+    return;
+  }
   if (p.pervox_eps) step_fused_kernel<T, true><<<grid, block, FusedGeom<T, true>::SMEM, st>>>(p, maps);
   else step_fused_kernel<T, false><<<grid, block, FusedGeom<T, false>::SMEM, st>>>(p, maps);
 }
 
+template <typename T, bool PV, bool STALL = false>
+static int set_fused_attr() {
+  return int(cudaFuncSetAttribute(step_fused_kernel<T, PV, STALL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(FusedGeom<T, PV>::SMEM)));
+}
+
 template <typename T>
 int prepare_fused_kernels() {
-  int e = 0;
-  e |= int(cudaFuncSetAttribute(step_fused_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                int(FusedGeom<T, true>::SMEM)));
-  e |= int(cudaFuncSetAttribute(step_fused_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                int(FusedGeom<T, false>::SMEM)));
-  return e;
+  return set_fused_attr<T, true>() | set_fused_attr<T, false>() | set_fused_attr<T, true, true>() |
+         set_fused_attr<T, false, true>();
 }
 
 template <typename T>

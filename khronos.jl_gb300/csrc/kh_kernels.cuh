@@ -205,9 +205,10 @@ struct HalfStepParams {
   int view_form;  // 2: the form for grids of more than one round of CTAs
 
   int* err;  // set to KH_ERR_TIMEOUT by a kernel whose bounded wait gave up
-  // Failure-detection test hook (0 in normal runs): nonzero launches the FP32
-  // LEAN TMA kernels' test instantiation, whose first ring stage expects 16
-  // bytes that never arrive, so its waits give up after 4096 polls.
+  // Failure-detection test hook (0 in normal runs): nonzero launches the FP32 test
+  // instantiation of the TMA kernels (LEAN, reduced-state, whole-step), whose first
+  // ring stage expects 16 bytes that never arrive, so its waits give up: after 4096
+  // polls, or 64 timed waits in the latter two.
   uint32_t stall_tx;
 };
 
@@ -289,6 +290,7 @@ struct FusedParams {
   long long n_tile_words;
   const uint32_t* cell_class;
   int* err;
+  uint32_t stall_tx;  // as in HalfStepParams
 };
 
 // Boxes: E (kTmaX + 16 bytes) × (kFusedRows + 1), H kTmaX × kFusedRows,

@@ -2072,7 +2072,7 @@ class Sim : public SimBase {
     if constexpr (sizeof(T) == 4) {
       const char* fv = std::getenv("KHRONOS_GB300_FUSED");
       if (!second_set_ok_ || !reduced_[0] || !reduced_[1] || pml_axis_[0] || pml_axis_[1] || pml_axis_[2] ||
-          d_.periodic || has_src_[1] || mu_[0] || stall_tx_ || (fv && std::string(fv) == "0"))
+          d_.periodic || has_src_[1] || mu_[0] || (fv && std::string(fv) == "0"))
         return KH_OK;
       const size_t field = size_t(total_ + pitch_) * sizeof(T);
       size_t free_b = 0, all_b = 0;
@@ -2152,6 +2152,7 @@ class Sim : public SimBase {
       p.n_tile_words = tbits_e_ ? (long long)((n_[2] + 63) / 64) * n_[1] * nxb_ : 0;
       p.cell_class = cls_;
       p.err = err_dev_;
+      p.stall_tx = stall_tx_;
       kh::launch_step_fused<T>(p, fused_maps_[from], st);
       ++launches;
     }
