@@ -40,7 +40,7 @@ KH_DBG_READER(dbg_read_kernels)
 template <typename T, int VN>
 struct PlaneLoads {
   T l0[VN], l1[VN], a2[VN], y0[VN], y2[VN];  // A0/A1 fresh plane, A2, y neighbours
-  T xn1, xn2;                                // x neighbours of A1/A2 for the edge lane
+  T xn1, xn2;                                // x neighbours of A1/A2 for the edge lanes
   T O[3][VN], m[3][VN];
   T t[3][VN], u[3][VN], w[3][VN], c3[VN];
   uint32_t cls[VN];
@@ -49,8 +49,8 @@ struct PlaneLoads {
 
 template <typename T, int VN, bool H, bool FULL>
 __device__ __forceinline__ void load_plane(const HalfStepParams<T>& p, PlaneLoads<T, VN>& L, int k,
-                                           long long row, int lane, bool lane_ok, bool pervox, bool fy,
-                                           bool anyfx, uint64_t tbits) {
+                                           long long row, int lane, bool row_end, bool lane_ok, bool pervox,
+                                           bool fy, bool anyfx, uint64_t tbits) {
   constexpr int s = H ? 1 : -1;
   const long long q = row + (long long)k * p.plane;
   vzero(L.l0); vzero(L.l1); vzero(L.a2); vzero(L.y0); vzero(L.y2);
@@ -72,7 +72,7 @@ __device__ __forceinline__ void load_plane(const HalfStepParams<T>& p, PlaneLoad
     vld_at(p.A[0], q + s * p.pitch, p.total, 3003, L.y0);
     vld_at(p.A[2], q + s * p.pitch, p.total, 3003, L.y2);
     if constexpr (H) {
-      if (lane == 31 && KH_IN(q + VN, p.total, 3004)) {
+      if (row_end && KH_IN(q + VN, p.total, 3004)) {
         L.xn1 = p.A[1][q + VN];
         L.xn2 = p.A[2][q + VN];
       }
@@ -121,8 +121,8 @@ __device__ __forceinline__ void load_plane(const HalfStepParams<T>& p, PlaneLoad
 // plane of A0/A1 in and out.
 template <typename T, int VN, bool H, bool CPML, bool FULL>
 __device__ __forceinline__ void compute_plane(const HalfStepParams<T>& p, PlaneLoads<T, VN>& L, int k,
-                                              long long row, int lane, bool lane_ok, int x0, int j,
-                                              bool fy, bool anyfx, const bool (&fxv)[VN],
+                                              long long row, int lane, bool row_end, bool lane_ok, int x0,
+                                              int j, bool fy, bool anyfx, const bool (&fxv)[VN],
                                               const AxisCoef<T> (&axv)[VN], const AxisCoef<T>& ay,
                                               T (&r0)[VN], T (&r1)[VN]) {
   const long long q = row + (long long)k * p.plane;
@@ -137,7 +137,7 @@ __device__ __forceinline__ void compute_plane(const HalfStepParams<T>& p, PlaneL
   if constexpr (H) {
     T n1 = __shfl_down_sync(0xffffffffu, cur1[0], 1);
     T n2 = __shfl_down_sync(0xffffffffu, L.a2[0], 1);
-    if (lane == 31) {
+    if (row_end) {
       n1 = L.xn1;
       n2 = L.xn2;
     }
@@ -261,6 +261,9 @@ __global__ void __launch_bounds__(32 * kBlockY, sizeof(T) == 4 ? kMinBlocks : 2)
   const int xb = blockIdx.x;
   const int x0 = (xb * 32 + lane) * VN;
   const bool lane_ok = x0 < p.nx;
+  // nobody in the warp has this lane's right neighbour: at the row's end that is the
+  // ring, the face across where x is periodic
+  const bool row_end = lane == 31 || x0 + VN >= p.nx;
   const int k0 = blockIdx.z * kPlanesPerCta;
   const int k1 = min(k0 + kPlanesPerCta, p.nz);
   const long long row = p.origin + (long long)j * p.pitch + x0;
@@ -294,14 +297,14 @@ __global__ void __launch_bounds__(32 * kBlockY, sizeof(T) == 4 ? kMinBlocks : 2)
     vld_at(p.A[1], q0, p.total, 3021, r1);
   }
   PlaneLoads<T, VN> A, B;
-  load_plane<T, VN, H, FULL>(p, A, k0, row, lane, lane_ok, pervox, fy, anyfx, tbits);
-  if (k0 + 1 < k1) load_plane<T, VN, H, FULL>(p, B, k0 + 1, row, lane, lane_ok, pervox, fy, anyfx, tbits);
+  load_plane<T, VN, H, FULL>(p, A, k0, row, lane, row_end, lane_ok, pervox, fy, anyfx, tbits);
+  if (k0 + 1 < k1) load_plane<T, VN, H, FULL>(p, B, k0 + 1, row, lane, row_end, lane_ok, pervox, fy, anyfx, tbits);
   for (int k = k0; k < k1; k += 2) {
-    compute_plane<T, VN, H, CPML, FULL>(p, A, k, row, lane, lane_ok, x0, j, fy, anyfx, fxv, axv, ay, r0, r1);
-    if (k + 2 < k1) load_plane<T, VN, H, FULL>(p, A, k + 2, row, lane, lane_ok, pervox, fy, anyfx, tbits);
+    compute_plane<T, VN, H, CPML, FULL>(p, A, k, row, lane, row_end, lane_ok, x0, j, fy, anyfx, fxv, axv, ay, r0, r1);
+    if (k + 2 < k1) load_plane<T, VN, H, FULL>(p, A, k + 2, row, lane, row_end, lane_ok, pervox, fy, anyfx, tbits);
     if (k + 1 < k1) {
-      compute_plane<T, VN, H, CPML, FULL>(p, B, k + 1, row, lane, lane_ok, x0, j, fy, anyfx, fxv, axv, ay, r0, r1);
-      if (k + 3 < k1) load_plane<T, VN, H, FULL>(p, B, k + 3, row, lane, lane_ok, pervox, fy, anyfx, tbits);
+      compute_plane<T, VN, H, CPML, FULL>(p, B, k + 1, row, lane, row_end, lane_ok, x0, j, fy, anyfx, fxv, axv, ay, r0, r1);
+      if (k + 3 < k1) load_plane<T, VN, H, FULL>(p, B, k + 3, row, lane, row_end, lane_ok, pervox, fy, anyfx, tbits);
     }
   }
 }
