@@ -356,7 +356,7 @@ template <typename T>
 int tma_resident_ctas();
 
 // Reduced-state half-step (kh_lean.cu) for the CUDA-path CPML stages; its maps
-// have boxes of kLeanY rows.  expand: the complete T, U, W from its state (o_kept: the
+// are the general kernel's.  expand: the complete T, U, W from its state (o_kept: the
 // array of T holds a copy of O where O is the state, see KeepArgs).
 template <typename T>
 void launch_half_step_lean(bool h_half, const HalfStepParams<T>& p, const TmaMaps& maps, void* stream);

@@ -1698,7 +1698,7 @@ class Sim : public SimBase {
       mark(s, 0);
       ph.view = view(1, s);
       ph.zplanes = reduced_[1] && !ph.full ? zplanes_[ph.view != 0] : general_zplanes_;
-      if (reduced_[1] && !ph.full) kh::launch_half_step_lean<T>(true, ph, lean_maps_h_, st);
+      if (reduced_[1] && !ph.full) kh::launch_half_step_lean<T>(true, ph, maps_h_, st);
       else if (use_tma_) kh::launch_half_step_tma<T>(true, ph, maps_h_, st);
       else kh::launch_half_step<T>(true, ph, st);
       ++launches;
@@ -1721,7 +1721,7 @@ class Sim : public SimBase {
       pe.full = (full_e_base || (src_e && !src_lean_ok_[0]) || complete(0, s)) ? 1 : 0;
       pe.view = view(0, s);
       pe.zplanes = reduced_[0] && !pe.full ? zplanes_[pe.view != 0] : general_zplanes_;
-      if (reduced_[0] && !pe.full) kh::launch_half_step_lean<T>(false, pe, lean_maps_e_, st);
+      if (reduced_[0] && !pe.full) kh::launch_half_step_lean<T>(false, pe, maps_e_, st);
       else if (use_tma_) kh::launch_half_step_tma<T>(false, pe, maps_e_, st);
       else kh::launch_half_step<T>(false, pe, st);
       ++launches;
@@ -2003,32 +2003,26 @@ class Sim : public SimBase {
     for (int v = 0; v < 3; ++v) lean_slots_[v] = sms_ * kh::lean_resident_ctas<T>(v);
     tma_slots_ = sms_ * kh::tma_resident_ctas<T>();
     const int hx = 16 / int(sizeof(T));
-    struct MapSet {
-      kh::TmaMaps *h, *e;
-      int cols, rows;
-    };
-    for (const MapSet& ms : {MapSet{&maps_h_, &maps_e_, kh::kTmaX, kh::kTmaY},
-                             MapSet{&lean_maps_h_, &lean_maps_e_, kh::kLeanX, kh::kLeanY}}) {
-      const cuuint32_t box_a[3] = {cuuint32_t(ms.cols + hx), cuuint32_t(ms.rows + 1), 1};
-      const cuuint32_t box_o[3] = {cuuint32_t(ms.cols), cuuint32_t(ms.rows), 1};
-      kh::TmaMaps &maps_h = *ms.h, &maps_e = *ms.e;
-      std::memset(&maps_h, 0, sizeof(maps_h));
-      std::memset(&maps_e, 0, sizeof(maps_e));
-      for (int c = 0; c < 3; ++c) {
-        kh_status st;
-        if ((st = encode_map(&maps_h.a[c], E_[c], box_a)) != KH_OK) return st;
-        if ((st = encode_map(&maps_h.o[c], H_[c], box_o)) != KH_OK) return st;
-        if (mu_[c] && (st = encode_map(&maps_h.m[c], mu_[c], box_o)) != KH_OK) return st;
-        if ((st = encode_map(&maps_e.a[c], H_[c], box_a)) != KH_OK) return st;
-        if ((st = encode_map(&maps_e.o[c], E_[c], box_o)) != KH_OK) return st;
-        if (eps_[c] && (st = encode_map(&maps_e.m[c], eps_[c], box_o)) != KH_OK) return st;
-        if (B_[c] && (st = encode_map(&maps_h.t[c], B_[c], box_o)) != KH_OK) return st;
-        if (UB_[c] && (st = encode_map(&maps_h.u[c], UB_[c], box_o)) != KH_OK) return st;
-        if (WB_[c] && (st = encode_map(&maps_h.w[c], WB_[c], box_o)) != KH_OK) return st;
-        if (D_[c] && (st = encode_map(&maps_e.t[c], D_[c], box_o)) != KH_OK) return st;
-        if (UD_[c] && (st = encode_map(&maps_e.u[c], UD_[c], box_o)) != KH_OK) return st;
-        if (WD_[c] && (st = encode_map(&maps_e.w[c], WD_[c], box_o)) != KH_OK) return st;
-      }
+    // one set of maps for the reduced-state and the general kernel
+    static_assert(kh::kTmaX == kh::kLeanX && kh::kTmaY == kh::kLeanY, "the tensor maps' boxes");
+    const cuuint32_t box_a[3] = {cuuint32_t(kh::kTmaX + hx), cuuint32_t(kh::kTmaY + 1), 1};
+    const cuuint32_t box_o[3] = {cuuint32_t(kh::kTmaX), cuuint32_t(kh::kTmaY), 1};
+    std::memset(&maps_h_, 0, sizeof(maps_h_));
+    std::memset(&maps_e_, 0, sizeof(maps_e_));
+    for (int c = 0; c < 3; ++c) {
+      kh_status st;
+      if ((st = encode_map(&maps_h_.a[c], E_[c], box_a)) != KH_OK) return st;
+      if ((st = encode_map(&maps_h_.o[c], H_[c], box_o)) != KH_OK) return st;
+      if (mu_[c] && (st = encode_map(&maps_h_.m[c], mu_[c], box_o)) != KH_OK) return st;
+      if ((st = encode_map(&maps_e_.a[c], H_[c], box_a)) != KH_OK) return st;
+      if ((st = encode_map(&maps_e_.o[c], E_[c], box_o)) != KH_OK) return st;
+      if (eps_[c] && (st = encode_map(&maps_e_.m[c], eps_[c], box_o)) != KH_OK) return st;
+      if (B_[c] && (st = encode_map(&maps_h_.t[c], B_[c], box_o)) != KH_OK) return st;
+      if (UB_[c] && (st = encode_map(&maps_h_.u[c], UB_[c], box_o)) != KH_OK) return st;
+      if (WB_[c] && (st = encode_map(&maps_h_.w[c], WB_[c], box_o)) != KH_OK) return st;
+      if (D_[c] && (st = encode_map(&maps_e_.t[c], D_[c], box_o)) != KH_OK) return st;
+      if (UD_[c] && (st = encode_map(&maps_e_.u[c], UD_[c], box_o)) != KH_OK) return st;
+      if (WD_[c] && (st = encode_map(&maps_e_.w[c], WD_[c], box_o)) != KH_OK) return st;
     }
     return KH_OK;
   }
@@ -2532,8 +2526,7 @@ class Sim : public SimBase {
   int sms_ = 1;
   int fused_slots_ = 1;  // SMs × resident whole-step CTAs per SM
   int lean_slots_[3] = {1, 1, 1}, tma_slots_ = 1;  // … reduced-state, general-kernel CTAs per SM
-  kh::TmaMaps maps_h_, maps_e_;            // kTmaY rows (general kernel)
-  kh::TmaMaps lean_maps_h_, lean_maps_e_;  // kLeanY rows (reduced-state kernel)
+  kh::TmaMaps maps_h_, maps_e_;
   // [E half, H half]: the reduced-state kernel takes this half's launches.  T, U
   // and W that follow from the rest of the state are then not kept up to date.
   bool reduced_[2] = {false, false};
