@@ -414,7 +414,9 @@ kh_status kh_debug_bounds(int64_t* count, int64_t* index, int32_t* site);
  * before prepare; estimate_memory, src/Memory.jl:120-251) and what it has
  * allocated (0 before prepare).  FP32 grids without CPML may add a second set of
  * E and H on top of the estimate, only while that is below 1/16 of the free
- * device memory and never for requests of a server. */
+ * device memory and never for requests of a server.  Grids without sources, poles
+ * and χ3 whose ε⁻¹ or μ⁻¹ is zero somewhere in the absorber add their cell classes
+ * (4 bytes per cell). */
 kh_status kh_sim_memory_bytes(const kh_sim* sim, int64_t* estimate, int64_t* allocated);
 
 /* State control. */

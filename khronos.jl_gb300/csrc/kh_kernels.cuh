@@ -388,6 +388,10 @@ struct KeepArgs {
 };
 template <typename T>
 void launch_keep_state(const KeepArgs<T>& a, int halves, bool from_t, void* stream);
+// Cells of the layers whose T does not follow from O (m⁻¹ = 0) marked as special in cls;
+// cls null: found set to 1 if there are any.
+template <typename T>
+void launch_dead_cells(const KeepArgs<T>& a, int halves, uint32_t* cls, int* found, void* stream);
 // A complete state against what the reduced one takes for granted in CPML cells
 // without special state: broken, W = m·T (own axis) or O = m·T (outside it) does not
 // hold to rounding; off_u against top_t, the largest |U - T| where only the next axis

@@ -491,26 +491,32 @@ void launch_expand_state(bool h_half, const HalfStepParams<T>& p, bool o_kept, v
 
 // O of the CPML cells where it is the state into the array of T, free there (KeepArgs):
 // one thread per cell of the absorber's layers.
+// Cell u of the layers: its indices and its place in the padded arrays.
+template <typename T>
+__device__ __forceinline__ long long layer_cell(const KeepArgs<T>& a, long long u, int (&at)[3]) {
+  int b = 0;
+  while (u >= a.first[b + 1]) ++b;
+  const long long e = u - a.first[b];
+  if (e <= 0xffffffffll) {  // 32-bit division wherever the index fits
+    const unsigned r = unsigned(e) / unsigned(a.dims[b][0]);
+    at[0] = a.start[b][0] + int(unsigned(e) - r * unsigned(a.dims[b][0]));
+    at[2] = a.start[b][2] + int(r / unsigned(a.dims[b][1]));
+    at[1] = a.start[b][1] + int(r % unsigned(a.dims[b][1]));
+  } else {
+    const long long r = e / a.dims[b][0];
+    at[0] = a.start[b][0] + int(e % a.dims[b][0]);
+    at[2] = a.start[b][2] + int(r / a.dims[b][1]);
+    at[1] = a.start[b][1] + int(r % a.dims[b][1]);
+  }
+  return a.origin + at[2] * a.plane + at[1] * a.pitch + at[0];
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) keep_state_kernel(const __grid_constant__ KeepArgs<T> a, bool from_t) {
   const KeepHalf<T>& h = a.half[blockIdx.y];
   for (long long u = blockIdx.x * 256ll + threadIdx.x; u < a.first[6]; u += gridDim.x * 256ll) {
-    int b = 0;
-    while (u >= a.first[b + 1]) ++b;
-    const long long e = u - a.first[b];
     int at[3];
-    if (e <= 0xffffffffll) {  // 32-bit division wherever the index fits
-      const unsigned r = unsigned(e) / unsigned(a.dims[b][0]);
-      at[0] = a.start[b][0] + int(unsigned(e) - r * unsigned(a.dims[b][0]));
-      at[2] = a.start[b][2] + int(r / unsigned(a.dims[b][1]));
-      at[1] = a.start[b][1] + int(r % unsigned(a.dims[b][1]));
-    } else {
-      const long long r = e / a.dims[b][0];
-      at[0] = a.start[b][0] + int(e % a.dims[b][0]);
-      at[2] = a.start[b][2] + int(r / a.dims[b][1]);
-      at[1] = a.start[b][1] + int(r % a.dims[b][1]);
-    }
-    const long long q = a.origin + at[2] * a.plane + at[1] * a.pitch + at[0];
+    const long long q = layer_cell(a, u, at);
     if (!KH_IN(q, a.total, 2151)) continue;
     if (h.tile_bits) {  // special cells keep their T
       const long long w = ((long long)(at[2] >> 6) * a.n[1] + at[1]) * a.nxb + (at[0] >> 6);
@@ -535,6 +541,34 @@ void launch_keep_state(const KeepArgs<T>& a, int halves, bool from_t, void* stre
   if (a.first[6] <= 0) return;
   const dim3 grid(unsigned(std::min<long long>((a.first[6] + 255) / 256, 1 << 30)), unsigned(halves));
   keep_state_kernel<T><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(a, from_t);
+}
+
+// Cells of the layers where O is the state and m⁻¹ = 0: T does not follow from a field
+// that is zero, so they keep it as special cells do.  Without cls: are there any?
+template <typename T>
+__global__ void __launch_bounds__(256) dead_cells_kernel(const __grid_constant__ KeepArgs<T> a, uint32_t* cls, int* found) {
+  const KeepHalf<T>& h = a.half[blockIdx.y];
+  for (long long u = blockIdx.x * 256ll + threadIdx.x; u < a.first[6]; u += gridDim.x * 256ll) {
+    int at[3];
+    const long long q = layer_cell(a, u, at);
+    if (!KH_IN(q, a.total, 2152)) continue;
+    bool dead = false;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const bool derived = !(at[c] < h.lo[c] || at[c] >= a.n[c] - h.hi[c]);
+      dead |= derived && h.m_inv[c] && h.m_inv[c][q] == T(0);
+    }
+    if (!dead) continue;
+    if (cls) atomicOr(cls + q, h.special);
+    else *found = 1;
+  }
+}
+
+template <typename T>
+void launch_dead_cells(const KeepArgs<T>& a, int halves, uint32_t* cls, int* found, void* stream) {
+  if (a.first[6] <= 0) return;
+  const dim3 grid(unsigned(std::min<long long>((a.first[6] + 255) / 256, 1 << 30)), unsigned(halves));
+  dead_cells_kernel<T><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(a, cls, found);
 }
 
 // What the reduced state takes for granted, checked on the complete T, U and W of a
@@ -696,6 +730,8 @@ template void launch_expand_state<float>(bool, const HalfStepParams<float>&, boo
 template void launch_expand_state<double>(bool, const HalfStepParams<double>&, bool, void*);
 template void launch_keep_state<float>(const KeepArgs<float>&, int, bool, void*);
 template void launch_keep_state<double>(const KeepArgs<double>&, int, bool, void*);
+template void launch_dead_cells<float>(const KeepArgs<float>&, int, uint32_t*, int*, void*);
+template void launch_dead_cells<double>(const KeepArgs<double>&, int, uint32_t*, int*, void*);
 template void launch_check_state<float>(bool, const HalfStepParams<float>&, StateCheck<float>*, void*);
 template void launch_check_state<double>(bool, const HalfStepParams<double>&, StateCheck<double>*, void*);
 template int prepare_lean_kernels<float>();

@@ -714,21 +714,7 @@ class Sim : public SimBase {
       KH_TRY(alloc_raw(nwords * sizeof(uint64_t), (void**)&tbits_e_, false));
       KH_TRY(alloc_raw(nwords * sizeof(uint64_t), (void**)&tbits_h_, false));
       KH_TRY(alloc_raw(sizeof(unsigned int), (void**)&region_flags, false));
-      kh::TileBitsArgs ta;
-      for (int a = 0; a < 3; ++a) {
-        ta.n[a] = n_[a];
-        ta.lo[a] = lo_[a];
-        ta.hi[a] = hi_[a];
-      }
-      ta.pitch = pitch_;
-      ta.plane = plane_;
-      ta.origin = origin_;
-      ta.nxb = nxb_;
-      ta.cls = cls_;
-      ta.bits_e = reinterpret_cast<unsigned long long*>(tbits_e_);
-      ta.bits_h = reinterpret_cast<unsigned long long*>(tbits_h_);
-      ta.region_flags = region_flags;
-      kh::launch_tile_bits(ta, cudaStreamLegacy);
+      kh::launch_tile_bits(tile_bits_args(region_flags), cudaStreamLegacy);
       ++launches;
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return fail(KH_ERR_CUDA, std::string("classification kernels: ") + cudaGetErrorString(e));
@@ -850,6 +836,7 @@ class Sim : public SimBase {
       reduced_[0] = !(msigd_[0] || msigd_[1] || msigd_[2]) && (!dispersive || disp_fix_);
       reduced_[1] = !(msigb_[0] || msigb_[1] || msigb_[2]);
     }
+    KH_TRY(keep_dead_cells());
     KH_TRY(prepare_fused());
     prepared_ = true;
     return KH_OK;
@@ -1064,13 +1051,11 @@ class Sim : public SimBase {
     // mid-run in a CPML cell of a half on the reduced state: W keeps the old
     // material's value for one step, which goes through the complete state
     const int half = kind == KH_MAT_MU_INV ? 1 : 0;
-    if (timestep_ > 0 && reduced_[half] && complete_[half] == kDerived) {
-      bool cpml = false;
-      for (int a = 0; a < 3; ++a) cpml = cpml || st[a] < lo_[a] || st[a] + dm[a] > n_[a] - hi_[a];
-      if (cpml) {
-        if (kh_status es = expand_state(half); es != KH_OK) return es;
-        complete_[half] = kOneStep;
-      }
+    bool cpml = false, zero = false;
+    for (int a = 0; a < 3; ++a) cpml = cpml || st[a] < lo_[a] || st[a] + dm[a] > n_[a] - hi_[a];
+    if (cpml && timestep_ > 0 && reduced_[half] && complete_[half] == kDerived) {
+      if (kh_status es = expand_state(half); es != KH_OK) return es;
+      complete_[half] = kOneStep;
     }
     std::vector<T> plane(size_t(dm[0]) * dm[1]);
     for (int k = 0; k < dm[2]; ++k) {
@@ -1078,13 +1063,14 @@ class Sim : public SimBase {
         for (int i = 0; i < dm[0]; ++i) {
           const T val = T(v[(size_t(k) * dm[1] + j) * dm[0] + i]);
           plane[size_t(j) * dm[0] + i] = val;
+          zero |= val == T(0);
           if (!host->empty()) (*host)[(size_t(st[2] + k) * n_[1] + (st[1] + j)) * n_[0] + (st[0] + i)] = val;
         }
       T* row0 = dst + origin_ + (long long)(st[2] + k) * plane_ + (long long)st[1] * pitch_ + st[0];
       KH_CUDA(cudaMemcpy2D(row0, size_t(pitch_) * sizeof(T), plane.data(), size_t(dm[0]) * sizeof(T),
                            size_t(dm[0]) * sizeof(T), size_t(dm[1]), cudaMemcpyHostToDevice));
     }
-    return KH_OK;
+    return zero && cpml && reduced_[half] ? keep_dead_cells() : KH_OK;
   }
 
   // Replace source `index`'s amplitudes (the cells it injects into stay the
@@ -2231,14 +2217,12 @@ class Sim : public SimBase {
     return KH_OK;
   }
 
-  // The copies of the halves in mask (bit 0: E, bit 1: H) that views are out of.
-  void launch_keep(int mask, bool from_t, cudaStream_t st) {
-    if (!(pml_axis_[0] || pml_axis_[1] || pml_axis_[2])) return;
-    kh::KeepArgs<T> a;
+  // The absorber's layers for the halves in mask (bit 0: E, bit 1: H); their number.
+  int keep_args(int mask, kh::KeepArgs<T>& a) const {
     std::memset(&a, 0, sizeof(a));
     int halves = 0;
     for (int h = 0; h < 2; ++h) {
-      if (!((mask >> h) & 1) || !reduced_[h] || !views_out_[h]) continue;
+      if (!((mask >> h) & 1)) continue;
       kh::KeepHalf<T>& k = a.half[halves++];
       for (int c = 0; c < 3; ++c) {
         k.O[c] = h ? H_[c] : E_[c];
@@ -2251,7 +2235,6 @@ class Sim : public SimBase {
       k.tile_bits = h ? tbits_h_ : tbits_e_;
       k.special = h ? kh::kSpecialH : kh::kSpecialE;
     }
-    if (!halves) return;
     a.nxb = nxb_;
     a.pitch = pitch_;
     a.plane = plane_;
@@ -2281,8 +2264,82 @@ class Sim : public SimBase {
       }
       a.first[b + 1] = a.first[b] + 1ll * a.dims[b][0] * a.dims[b][1] * a.dims[b][2];
     }
+    return halves;
+  }
+
+  // The copies of the halves in mask that views are out of.
+  void launch_keep(int mask, bool from_t, cudaStream_t st) {
+    for (int h = 0; h < 2; ++h)
+      if (!reduced_[h] || !views_out_[h]) mask &= ~(1 << h);
+    kh::KeepArgs<T> a;
+    const int halves = keep_args(mask, a);
+    if (!halves || a.first[6] == 0) return;
     kh::launch_keep_state<T>(a, halves, from_t, st);
     ++launches;
+  }
+
+  // Cells of the absorber with m⁻¹ = 0 become special cells (launch_dead_cells); also
+  // called when a material is set to 0 between steps, with T then up to date.
+  kh_status keep_dead_cells() {
+    int mask = 0;
+    for (int h = 0; h < 2; ++h)
+      if (reduced_[h] && (h ? mu_[0] : eps_[0])) mask |= 1 << h;
+    kh::KeepArgs<T> a;
+    const int halves = keep_args(mask, a);
+    if (!halves || a.first[6] == 0) return KH_OK;
+    struct Flags {
+      int found;
+      unsigned int regions;
+    } *dev = nullptr, got{};
+    KH_CUDA(kh_host::dev_alloc((void**)&dev, sizeof(Flags), cudaStreamLegacy));
+    cudaError_t e = cudaMemsetAsync(dev, 0, sizeof(Flags), cudaStreamLegacy);
+    if (e == cudaSuccess) {
+      kh::launch_dead_cells<T>(a, halves, nullptr, &dev->found, cudaStreamLegacy);
+      ++launches;
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(&got, dev, sizeof(Flags), cudaMemcpyDeviceToHost);
+    kh_status st = KH_OK;
+    if (e == cudaSuccess && got.found) {
+      if (!cls_) {
+        const size_t words = size_t((n_[2] + 63) / 64) * n_[1] * nxb_ * sizeof(uint64_t);
+        if ((st = alloc_raw(size_t(total_) * sizeof(uint32_t), (void**)&cls_, false)) == KH_OK &&
+            (st = alloc_raw(words, (void**)&tbits_e_, false)) == KH_OK)
+          st = alloc_raw(words, (void**)&tbits_h_, false);
+        // captured steps have no classes
+        for (auto& g : graphs_) cudaGraphExecDestroy(g.exec);
+        graphs_.clear();
+      }
+      if (st == KH_OK) {
+        kh::launch_dead_cells<T>(a, halves, cls_, nullptr, cudaStreamLegacy);
+        kh::launch_tile_bits(tile_bits_args(&dev->regions), cudaStreamLegacy);
+        launches += 2;
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+      }
+    }
+    kh_host::dev_free(dev, cudaStreamLegacy);
+    if (st != KH_OK) return st;
+    if (e != cudaSuccess) return fail(KH_ERR_CUDA, std::string("cells of zero material: ") + cudaGetErrorString(e));
+    return KH_OK;
+  }
+
+  kh::TileBitsArgs tile_bits_args(unsigned int* region_flags) const {
+    kh::TileBitsArgs ta;
+    for (int a = 0; a < 3; ++a) {
+      ta.n[a] = n_[a];
+      ta.lo[a] = lo_[a];
+      ta.hi[a] = hi_[a];
+    }
+    ta.pitch = pitch_;
+    ta.plane = plane_;
+    ta.origin = origin_;
+    ta.nxb = nxb_;
+    ta.cls = cls_;
+    ta.bits_e = reinterpret_cast<unsigned long long*>(tbits_e_);
+    ta.bits_h = reinterpret_cast<unsigned long long*>(tbits_h_);
+    ta.region_flags = region_flags;
+    return ta;
   }
 
   // The copies that the next call starts from (from_t: out of the complete state).
