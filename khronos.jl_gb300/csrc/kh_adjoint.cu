@@ -85,8 +85,6 @@ __global__ void __launch_bounds__(kRedThreads) overlap_final_kernel(const double
   if (threadIdx.x == 0) out[f] = s;
 }
 
-// Squared norm Σ|F|² of one DFT array (all cells and frequencies): block b
-// sums its contiguous chunk.
 // Σ|F|² of up to kNormBatch monitors in one launch: blocks first[m] … first[m+1] - 1
 // take monitor m's chunks, then one block per monitor adds them in order.  A run
 // under a decay criterion reads these after every monitor update; with two launches

@@ -16,10 +16,13 @@
 // ring of kFusedStages.  The arithmetic is that of the half-step kernel, bit for
 // bit.
 //
-// Bound by memory and the work on the halo (8/7 of the rows, 64/56 to 64/60 of
-// the columns for H).  216×200×168, 100 steps, against half-step launches:
-// 9.86 to 7.26 ms with a uniform ε (4.8 TB/s on 12 words a cell and step), 11.2 to
-// 8.55 with per-voxel ε.
+// Bound by memory and the work on the halo (8/7 of the rows, 64/32 to 64/60 of
+// the columns for H).  µs a step of 216×200×168 against half-steps: dipole 106 to 71
+// with a uniform ε (4.9 TB/s on 12 words a cell), 117 to 85 with per-voxel ε; a current
+// plane, which flags a segment of every row, 122 to 90 and 132 to 101.  Over 138 closed
+// boxes (20 to 400 cells an axis) half-steps were faster on few, all 60 to 64 cells
+// wide (two half-empty column tiles): 62×150×150 30.4 against 27.5, 64×128×128 24.7
+// against 23.6, 64×300×300 90 against 109.
 //
 // Every mbarrier wait is bounded, as in kh_lean.cu.
 #include <cuda.h>

@@ -7,8 +7,9 @@
 //   with origin = ((ny + 2) + 1) * pitch + XOFF and XOFF = 32 bytes of
 //   elements (xoff<T>()), so x = 0 of every row starts a 32-byte sector (a
 //   row segment of 64 cells covers whole sectors) and the row pitch is a
-//   multiple of 128 bytes.  The ring i,j,k in {-1, n} (and the row padding)
-//   is never written: it is the reference's zero ghost layer / staggered wall.
+//   multiple of 128 bytes.  The ring i,j,k in {-1, n} (and the row padding) is the
+//   reference's zero ghost layer / staggered wall: only periodic axes write their
+//   part of it.
 #pragma once
 
 #include <cuda.h>  // CUtensorMap (descriptors are encoded through the runtime's driver entry point)
@@ -234,9 +235,9 @@ constexpr int kTmaMinBlocks = KH_TMA_MIN_BLOCKS;
 // Reduced-state half-step (kh_lean.cu): tile of kLeanX × kLeanY cells, 8 bytes of
 // FP32 (16 of FP64) cells per thread, ring stages, resident CTAs per SM it is
 // compiled for, and how many planes ahead a lane in the x-CPML fetches its
-// auxiliaries into L2.  Measured on whole runs (ms: waveguide 320×192×128, 96
-// steps / closed box 216×200×168, 100 steps / 64³, 256 steps; this choice 15.99 /
-// 9.72 / 3.55): 4 FP32 cells per thread 16.83 / 9.81 / 3.98; five CTAs per SM
+// auxiliaries into L2.  Measured when the kernel was new, on whole runs in half-steps
+// (ms: waveguide 320×192×128, 96 steps / closed box 216×200×168, 100 steps / 64³, 256
+// steps; this choice 15.99 / 9.72 / 3.55 then, 14.95 / 10.55 / 3.29 now): 4 FP32 cells per thread 16.83 / 9.81 / 3.98; five CTAs per SM
 // 16.22 / 10.21 / 3.55; two stages 15.99 / 10.08 / 3.57; 128 × 4 tiles 17.18 / 9.87 /
 // 5.09; 128 × 2 16.85 / 9.65 / 4.97; 64 × 2 16.31 / 9.78 / 3.75.
 constexpr int kLeanX = 64;
@@ -264,7 +265,7 @@ struct alignas(128) TmaMaps {
 };
 
 // Whole-step kernel (kh_fused.cu): 8 rows of threads (a halo row and 7 owned),
-// ring stages, resident CTAs per SM, owned columns at most.  Two stages are in use
+// ring stages, resident CTAs per SM (one more with a uniform ε), owned columns at most.  Two stages are in use
 // while a plane is computed; with a fourth fewer CTAs fit (216×200×168 with per-voxel
 // ε, 100 steps: 2 / 3 / 4 stages 9.87 / 8.56 / 8.71 ms).
 constexpr int kFusedRows = 8;

@@ -9,7 +9,7 @@
 // with their x/y halo, updated components, m⁻¹).
 //
 // What bounds it: plain tiles run at the memory's rate (216×200×168 FP32 without
-// CPML: 48 µs a half-step for 262 MB, 5.5 TB/s); tiles in the CPML by the latency
+// CPML, which whole steps take by default: 48 µs a half-step for 262 MB, 5.5 TB/s); tiles in the CPML by the latency
 // of a plane (their auxiliaries' loads, then update, store and barrier) and its
 // instructions.  Against the complete cascade (T, U, W stored for every CPML cell)
 // a 320×192×128 step moves 757 instead of 978 MB, in 42 + 50 M instead of 64 + 66 M
@@ -70,9 +70,10 @@ __global__ void __launch_bounds__(kLeanThreads, (VIEW == 2 ? kLeanMinBlocks<T> -
   constexpr int VN = kLeanVN;
   static_assert(VN == 2, "paired loads of the class words");
   // Rows in update_row's branch-free forms, except in FP32 with per-voxel m⁻¹, where
-  // their longer live ranges spill at six CTAs per SM (320×192×128, 96 steps: 15.96 ms
-  // with update_cells in both halves, 15.37 with this choice, 15.73 with update_row in
-  // both; FP64 240×144×96, where a branch costs both sides' arithmetic, 17.9 to 13.0).
+  // their longer live ranges spill at six CTAs per SM (320×192×128, 96 steps, when it was
+  // chosen: 15.96 ms with update_cells in both halves, 15.37 with this choice, 15.73 with
+  // update_row in both; FP64 240×144×96, where a branch costs both sides' arithmetic, 17.9
+  // to 13.0).
   constexpr bool kRow = sizeof(T) == 8 || !PV;
   constexpr int LPR = kLeanX / VN;  // lanes per tile row
   using PK = Pack<T, VN>;
