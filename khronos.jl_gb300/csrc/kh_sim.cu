@@ -680,7 +680,9 @@ class Sim : public SimBase {
     // Cell classes and the per-row-segment plane bitmasks (word (k/64, j, xb),
     // bit k%64), computed on the device from the material arrays and the
     // source table.
-    unsigned int* region_flags = nullptr;
+    // the error word and what the device finds out about the cells, read back at once
+    KH_TRY(alloc_raw(sizeof(PrepFlags), (void**)&err_dev_, false));
+    PrepFlags* flags = reinterpret_cast<PrepFlags*>(err_dev_);
     if (anySpecialE || anySpecialH) {
       KH_TRY(alloc_raw(size_t(total_) * sizeof(uint32_t), (void**)&cls_, false));
       kh::ClassifyArgs<T> ca;
@@ -713,8 +715,7 @@ class Sim : public SimBase {
       const size_t nwords = size_t((n_[2] + 63) / 64) * n_[1] * nxb_;
       KH_TRY(alloc_raw(nwords * sizeof(uint64_t), (void**)&tbits_e_, false));
       KH_TRY(alloc_raw(nwords * sizeof(uint64_t), (void**)&tbits_h_, false));
-      KH_TRY(alloc_raw(sizeof(unsigned int), (void**)&region_flags, false));
-      kh::launch_tile_bits(tile_bits_args(region_flags), cudaStreamLegacy);
+      kh::launch_tile_bits(tile_bits_args(&flags->regions), cudaStreamLegacy);
       ++launches;
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return fail(KH_ERR_CUDA, std::string("classification kernels: ") + cudaGetErrorString(e));
@@ -767,7 +768,6 @@ class Sim : public SimBase {
       KH_CUDA(cudaEventCreateWithFlags(&ev_in_, cudaEventDisableTiming));
       KH_CUDA(cudaEventCreateWithFlags(&ev_out_, cudaEventDisableTiming));
     }
-    KH_TRY(alloc_raw(sizeof(int), (void**)&err_dev_, false));
     // Half-step kernel: TMA-staged unless KHRONOS_GB300_KERNEL=simt selects the
     // register-pipelined one.
     const char* kv = std::getenv("KHRONOS_GB300_KERNEL");
@@ -779,16 +779,22 @@ class Sim : public SimBase {
     if (const char* xv = std::getenv("KHRONOS_GB300_XPREFETCH")) xprefetch_ = std::min(2, std::max(0, std::atoi(xv)));
     if (const char* dv = std::getenv("KHRONOS_GB300_XPF_DIST")) xpf_dist_ = std::min(8, std::max(1, std::atoi(dv)));
     if (const char* sv = std::getenv("KHRONOS_GB300_TEST_STALL")) stall_tx_ = std::string(sv) == "1" ? 16u : 0u;
+    if (use_tma_ && d_.semantics == KH_SEM_CPML) {  // where a half may be on the reduced state
+      kh::KeepArgs<T> a;
+      const int halves = keep_args((eps_[0] ? 1 : 0) | (mu_[0] ? 2 : 0), a);
+      if (halves && a.first[6] > 0) {
+        kh::launch_dead_cells<T>(a, halves, nullptr, &flags->dead, cudaStreamLegacy);
+        ++launches;
+        KH_CUDA(cudaGetLastError());
+      }
+    }
     // the zeroing and uploads above ran on the legacy default stream; wait for
     // them only (work of other simulations on non-blocking streams goes on)
     KH_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
-    special_in_region_[0] = special_in_region_[1] = false;
-    if (region_flags) {
-      unsigned int rf = 0;
-      KH_CUDA(cudaMemcpy(&rf, region_flags, sizeof(rf), cudaMemcpyDeviceToHost));
-      special_in_region_[0] = (rf & 1u) != 0;
-      special_in_region_[1] = (rf & 2u) != 0;
-    }
+    PrepFlags got;
+    KH_CUDA(cudaMemcpy(&got, flags, sizeof(got), cudaMemcpyDeviceToHost));
+    special_in_region_[0] = (got.regions & 1u) != 0;
+    special_in_region_[1] = (got.regions & 2u) != 0;
     // χ3 and pole cells updated by the LEAN E launch plus the dispersive-cell
     // pass, unless something else needs the FULL launch anyway (material
     // conductivity, the CPU-path semantics with special cells in CPML, or a
@@ -836,7 +842,7 @@ class Sim : public SimBase {
       reduced_[0] = !(msigd_[0] || msigd_[1] || msigd_[2]) && (!dispersive || disp_fix_);
       reduced_[1] = !(msigb_[0] || msigb_[1] || msigb_[2]);
     }
-    KH_TRY(keep_dead_cells());
+    if (got.dead) KH_TRY(keep_dead_cells());
     KH_TRY(prepare_fused());
     prepared_ = true;
     return KH_OK;
@@ -920,7 +926,7 @@ class Sim : public SimBase {
       const int64_t cnt = int64_t(m.dims[0]) * m.dims[1] * m.dims[2] * m.nf * int64_t(sizeof(Cplx<T>));
       b += cnt * (sizeof(T) == 4 ? 2 : 1);
     }
-    b += 2 * int64_t(table_capacity() * sizeof(Cplx<T>)) + int64_t(sizeof(int));
+    b += 2 * int64_t(table_capacity() * sizeof(Cplx<T>)) + int64_t(sizeof(PrepFlags));
     for (auto& h : hists_) b += h.ncell * h.cap * int64_t(sizeof(T));
     return b;
   }
@@ -2278,8 +2284,8 @@ class Sim : public SimBase {
     ++launches;
   }
 
-  // Cells of the absorber with m⁻¹ = 0 become special cells (launch_dead_cells); also
-  // called when a material is set to 0 between steps, with T then up to date.
+  // Cells of the absorber with m⁻¹ = 0 become special cells (launch_dead_cells), at
+  // prepare and when a material is set to 0 between steps, T then being up to date.
   kh_status keep_dead_cells() {
     int mask = 0;
     for (int h = 0; h < 2; ++h)
@@ -2287,42 +2293,29 @@ class Sim : public SimBase {
     kh::KeepArgs<T> a;
     const int halves = keep_args(mask, a);
     if (!halves || a.first[6] == 0) return KH_OK;
-    struct Flags {
-      int found;
-      unsigned int regions;
-    } *dev = nullptr, got{};
-    KH_CUDA(kh_host::dev_alloc((void**)&dev, sizeof(Flags), cudaStreamLegacy));
-    cudaError_t e = cudaMemsetAsync(dev, 0, sizeof(Flags), cudaStreamLegacy);
-    if (e == cudaSuccess) {
-      kh::launch_dead_cells<T>(a, halves, nullptr, &dev->found, cudaStreamLegacy);
-      ++launches;
-      e = cudaGetLastError();
+    if (!cls_) {
+      const size_t words = size_t((n_[2] + 63) / 64) * n_[1] * nxb_ * sizeof(uint64_t);
+      if (kh_status st = alloc_raw(words, (void**)&tbits_e_, false); st != KH_OK) return st;
+      if (kh_status st = alloc_raw(words, (void**)&tbits_h_, false); st != KH_OK) return st;
+      if (kh_status st = alloc_raw(size_t(total_) * sizeof(uint32_t), (void**)&cls_, false); st != KH_OK) return st;
+      // captured steps have no classes
+      for (auto& g : graphs_) cudaGraphExecDestroy(g.exec);
+      graphs_.clear();
     }
-    if (e == cudaSuccess) e = cudaMemcpy(&got, dev, sizeof(Flags), cudaMemcpyDeviceToHost);
-    kh_status st = KH_OK;
-    if (e == cudaSuccess && got.found) {
-      if (!cls_) {
-        const size_t words = size_t((n_[2] + 63) / 64) * n_[1] * nxb_ * sizeof(uint64_t);
-        if ((st = alloc_raw(size_t(total_) * sizeof(uint32_t), (void**)&cls_, false)) == KH_OK &&
-            (st = alloc_raw(words, (void**)&tbits_e_, false)) == KH_OK)
-          st = alloc_raw(words, (void**)&tbits_h_, false);
-        // captured steps have no classes
-        for (auto& g : graphs_) cudaGraphExecDestroy(g.exec);
-        graphs_.clear();
-      }
-      if (st == KH_OK) {
-        kh::launch_dead_cells<T>(a, halves, cls_, nullptr, cudaStreamLegacy);
-        kh::launch_tile_bits(tile_bits_args(&dev->regions), cudaStreamLegacy);
-        launches += 2;
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
-      }
-    }
-    kh_host::dev_free(dev, cudaStreamLegacy);
-    if (st != KH_OK) return st;
+    kh::launch_dead_cells<T>(a, halves, cls_, nullptr, cudaStreamLegacy);
+    kh::launch_tile_bits(tile_bits_args(&reinterpret_cast<PrepFlags*>(err_dev_)->regions), cudaStreamLegacy);
+    launches += 2;
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e != cudaSuccess) return fail(KH_ERR_CUDA, std::string("cells of zero material: ") + cudaGetErrorString(e));
     return KH_OK;
   }
+
+  struct PrepFlags {
+    int err;               // what err_dev_ points at
+    unsigned int regions;  // TileBitsArgs::region_flags
+    int dead;              // launch_dead_cells found some
+  };
 
   kh::TileBitsArgs tile_bits_args(unsigned int* region_flags) const {
     kh::TileBitsArgs ta;
