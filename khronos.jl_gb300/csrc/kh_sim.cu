@@ -1195,6 +1195,7 @@ class Sim : public SimBase {
     KH_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     timestep_ = 0;
     sources_active_ = true;
+    ring_due_ = ring2_;
     complete_[0] = complete_[1] = kDerived;
     stay_complete();
     return KH_OK;
@@ -1235,6 +1236,7 @@ class Sim : public SimBase {
     }
     timestep_ = hdr[0];
     sources_active_ = (hdr[1] & 1) != 0;
+    ring_due_ = true;
     return check_imported();
   }
 
@@ -1661,7 +1663,7 @@ class Sim : public SimBase {
       return (first && s == 0 ? kh::kViewRestore : 0u) | (last && s == nb - 1 ? kh::kViewKeep : 0u);
     };
     // … and what may have been written outside the grid goes into the second set, too
-    const bool mirror = first && (views_out_[0] || views_out_[1]);
+    const bool mirror = whole && nb > 1 && ((first && (views_out_[0] || views_out_[1])) || ring_due_);
     auto issue_all = [&](cudaStream_t st) {
     for (int s = 0; s < nb; ++s) {
       // two whole steps, into the second set and back
@@ -1741,7 +1743,7 @@ class Sim : public SimBase {
       sig.push_back(nb);
       sig.push_back(b);
       sig.push_back(complete_[0] + 4 * complete_[1] + 16 * int(view(0, 0) | view(0, nb - 1)) +
-                    64 * int(view(1, 0) | view(1, nb - 1)) + (whole && mirror ? 256 : 0));
+                    64 * int(view(1, 0) | view(1, nb - 1)) + (mirror ? 256 : 0));
       for (int q = 0; q < nb; ++q) {
         const StepPlan& P = plan[q];
         sig.push_back(P.sa ? 1 : 0);
@@ -1810,6 +1812,10 @@ class Sim : public SimBase {
     batch_recorded_ = true;
     last_stream_ = stream;
     timestep_ += nb;
+    if (mirror) {
+      ring_due_ = false;
+      ring2_ = true;
+    }
     for (int h = 0; h < 2; ++h)
       if (complete_[h] == kOneStep) complete_[h] = kDerived;
     if (timing) {
@@ -2597,6 +2603,8 @@ class Sim : public SimBase {
   kh::FusedMaps fused_maps_[2];
   int fused_zplanes_ = 1, fused_w_ = kh::kFusedW;
   int cur_ = 0;
+  // set 1's ring may hold something, is to be copied from set 0 (a state imported, or zeroed)
+  bool ring2_ = false, ring_due_ = false;
 
   std::vector<void*> allocs_;
   std::vector<std::pair<void*, size_t>> state_;

@@ -165,3 +165,45 @@ def test_wall_layers_of_a_closed_box(kh, gpu_lib, monkeypatch, n):
     assert a.launches < b.launches  # whole steps were taken
     a.close()
     b.close()
+
+
+def test_wall_layers_of_an_imported_state(kh, gpu_lib, monkeypatch):
+    """The ring is part of a state: imported, it acts on every step without any view, and a
+    reset clears it from every step."""
+    import torch
+
+    from khronos_gb300.device import GpuSim
+
+    n = (61, 9, 14)
+    sp = _spec(kh, "f32", n, (0, 0, 0))
+    sp.materials = [m for m in sp.materials if m[0] == 0]
+    sp.sources = [s for s in sp.sources if s.component < 3]
+    first = GpuSim(sp, lib=gpu_lib)
+    first.step(6)
+    first.synchronize()
+    rng = np.random.default_rng(8)
+    for c in range(3):
+        v = first.field_view(c)
+        for ax in range(3):
+            if v.shape[ax] > n[ax]:
+                w = v.select(ax, n[ax])
+                w.copy_(torch.as_tensor(rng.standard_normal(tuple(w.shape)), device=v.device, dtype=v.dtype))
+    torch.cuda.synchronize()
+    blob = first.export_state()
+    first.close()
+    a = GpuSim(sp, lib=gpu_lib)
+    monkeypatch.setenv("KHRONOS_GB300_FUSED", "0")
+    b = GpuSim(sp, lib=gpu_lib)
+    for g in (a, b):
+        g.import_state(blob)
+        g.step(1)
+        g.step(12)
+    for c in range(6):
+        assert np.array_equal(a.field(c), b.field(c)), c
+    for g in (a, b):
+        g.reset()
+        g.step(12)
+    for c in range(6):
+        assert np.array_equal(a.field(c), b.field(c)), c
+    a.close()
+    b.close()
