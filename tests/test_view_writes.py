@@ -207,3 +207,42 @@ def test_wall_layers_of_an_imported_state(kh, gpu_lib, monkeypatch):
         assert np.array_equal(a.field(c), b.field(c)), c
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("pml", [(5, 4, 3), (0, 0, 0)])
+def test_bounds(kh, gpu_lib, pml):
+    """The bounds-checked build: no index out of range in the steps that mind views, the
+    copies outside of steps, the import check and the ring, and the same bits."""
+    import ctypes as C
+
+    from khronos_gb300 import _abi, build
+    from khronos_gb300.device import GpuSim
+
+    checked = _abi.load(build.build(bounds=True))
+    n = (71, 21, 18)
+    out = []
+    c, i, s = C.c_int64(), C.c_int64(), C.c_int32()
+    for lib in (gpu_lib, checked):
+        if lib is checked:
+            assert lib.kh_debug_bounds(C.byref(c), C.byref(i), C.byref(s)) == 0
+        sp = _spec(kh, "f32", n, pml)
+        if pml[0] == 0:  # whole steps
+            sp.materials = [m for m in sp.materials if m[0] == 0]
+            sp.sources = [q for q in sp.sources if q.component < 3]
+        else:
+            sp.materials[0][2][:9, :3] = 0.0
+        g = GpuSim(sp, lib=lib)
+        g.step(9)
+        _write(g, 1, n, 2.0 ** -6)
+        g.step(4)
+        blob = g.export_state()
+        g.update_material_box(0, 1, (0, 0, 0), np.full((n[0], 3, n[2]), 0.75))
+        g.step(1)
+        g.import_state(blob)
+        g.step(5)
+        out.append([g.field(q) for q in range(6)])
+        g.close()
+    assert checked.kh_debug_bounds(C.byref(c), C.byref(i), C.byref(s)) == 0
+    assert c.value == 0, (i.value, s.value)
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
