@@ -14,10 +14,11 @@
 // five, three instead of seven along an edge, six instead of nine in a corner.
 //
 // The operations are written with explicit roundings (no contraction left to
-// the compiler), so every kernel and every form of a row gives the same bits.  A
-// damped O is fma(m, B·d, A·O): with the factors A = B = 1 of a cell outside the
-// absorber that is the plain update, so such cells need no select (with
-// fma(A, O, m·B·d) they were rounded once more, in some forms only).
+// the compiler).  A damped O is fma(A, O, m·(B·d)): one rounding at the size of O a
+// step (fma(m, B·d, A·O) has two; FP32 fluxes of 64³ runs of 173 steps were then up to
+// 1.3e-6 off instead of 4.7e-7).  A plain O is fma(m, d, O) in every kernel and every
+// form of a row, so they give the same bits, but for one: FP64 rows beside the x-CPML
+// (row_o).
 #pragma once
 
 #include "kh_cell.cuh"
@@ -86,7 +87,7 @@ __device__ __forceinline__ void red_component(const RedAxis<T>& o, const RedAxis
       O = fma_rn(m, fma_rn(o.op, tn, -mul_rn(o.om, t)), O);
       t = tn;
     } else {
-      O = fma_rn(m, x, mul_rn(A, O));
+      O = fma_rn(A, O, mul_rn(m, x));
     }
   } else if (o.f) {
     const T tn = add_rn(t, d);
@@ -127,13 +128,13 @@ __device__ __forceinline__ void update_cells(const bool (&fx)[VN], bool anyfx, c
         const T un = fma_rn(ry.a, u.c[0].v[v], mul_rn(ry.b, K.c[0].v[v]));
         const T d = sub_rn(un, u.c[0].v[v]);
         u.c[0].v[v] = un;
-        O.c[0].v[v] = fma_rn(m.c[0].v[v], mul_rn(rz.b, d), mul_rn(rz.a, O.c[0].v[v]));
+        O.c[0].v[v] = fma_rn(rz.a, O.c[0].v[v], mul_rn(m.c[0].v[v], mul_rn(rz.b, d)));
       }
     } else {
       const T A = ry.f ? ry.a : rz.a, B = ry.f ? ry.b : rz.b;
 #pragma unroll
       for (int v = 0; v < VN; ++v)
-        O.c[0].v[v] = fma_rn(m.c[0].v[v], mul_rn(B, K.c[0].v[v]), mul_rn(A, O.c[0].v[v]));
+        O.c[0].v[v] = fma_rn(A, O.c[0].v[v], mul_rn(m.c[0].v[v], mul_rn(B, K.c[0].v[v])));
     }
     // component y: own axis y, damped along z; component z the other way
 #pragma unroll
@@ -150,7 +151,7 @@ __device__ __forceinline__ void update_cells(const bool (&fx)[VN], bool anyfx, c
       } else {
 #pragma unroll
         for (int v = 0; v < VN; ++v)
-          O.c[c].v[v] = fma_rn(m.c[c].v[v], mul_rn(d.b, K.c[c].v[v]), mul_rn(d.a, O.c[c].v[v]));
+          O.c[c].v[v] = fma_rn(d.a, O.c[c].v[v], mul_rn(m.c[c].v[v], mul_rn(d.b, K.c[c].v[v])));
       }
     }
   } else if (!(ry.f || rz.f)) {
@@ -159,9 +160,11 @@ __device__ __forceinline__ void update_cells(const bool (&fx)[VN], bool anyfx, c
       const AxisCoef<T> x = xt[v];  // a, b, 1-σ, 1+σ
       const T tn = add_rn(t.c[0].v[v], K.c[0].v[v]);
       const T o0 = fma_rn(m.c[0].v[v], fma_rn(x.op, tn, -mul_rn(x.ir, t.c[0].v[v])), O.c[0].v[v]);
+      const T o1 = fma_rn(x.s, O.c[1].v[v], mul_rn(m.c[1].v[v], mul_rn(x.om, K.c[1].v[v])));
+      const T o2 = fma_rn(x.s, O.c[2].v[v], mul_rn(m.c[2].v[v], mul_rn(x.om, K.c[2].v[v])));
       O.c[0].v[v] = fx[v] ? o0 : fma_rn(m.c[0].v[v], K.c[0].v[v], O.c[0].v[v]);
-      O.c[1].v[v] = fma_rn(m.c[1].v[v], mul_rn(x.om, K.c[1].v[v]), mul_rn(x.s, O.c[1].v[v]));
-      O.c[2].v[v] = fma_rn(m.c[2].v[v], mul_rn(x.om, K.c[2].v[v]), mul_rn(x.s, O.c[2].v[v]));
+      O.c[1].v[v] = fx[v] ? o1 : fma_rn(m.c[1].v[v], K.c[1].v[v], O.c[1].v[v]);
+      O.c[2].v[v] = fx[v] ? o2 : fma_rn(m.c[2].v[v], K.c[2].v[v], O.c[2].v[v]);
       t.c[0].v[v] = fx[v] ? tn : t.c[0].v[v];
     }
   } else {
@@ -174,6 +177,17 @@ __device__ __forceinline__ void update_cells(const bool (&fx)[VN], bool anyfx, c
       red_component(rz, rx, ry, K.c[2].v[v], m.c[2].v[v], O.c[2].v[v], t.c[2].v[v], u.c[2].v[v]);
     }
   }
+}
+
+// O of a cell that only the x-CPML may damp (f; w = B·d, and A = 1, w = d outside it).
+// FP32 selects the operands of one multiply-add (160×160×96 with uniform materials 64.2 to
+// 64.5 µs a step; selecting the result 64.8).  FP64, bound by arithmetic, leaves plain cells
+// fma(1, O, m·d), one rounding more at 2⁻⁵³ (with selects 128×96×96 145.8 to 150.5 µs).
+template <bool WX, typename T>
+__device__ __forceinline__ T row_o(bool f, T A, T O, T m, T w) {
+  if constexpr (!WX) return fma_rn(m, w, O);
+  else if constexpr (sizeof(T) == 8) return fma_rn(A, O, mul_rn(m, w));
+  else return fma_rn(f ? A : m, f ? O : w, f ? mul_rn(m, w) : O);
 }
 
 // Update of VN cells of a row without special cells, compiled for the CPMLs the
@@ -207,7 +221,7 @@ __device__ __forceinline__ void update_row(const bool (&fx)[VN], const AxisCoef<
       const T A = FZ ? za : ry.a, B = FZ ? zb : ry.b;
       const T w = FY || FZ ? mul_rn(B, d) : d;
       const T o = O.c[0].v[v], mm = m.c[0].v[v], tt = t.c[0].v[v];
-      T r = FY || FZ ? fma_rn(mm, w, mul_rn(A, o)) : fma_rn(mm, w, o);
+      T r = FY || FZ ? fma_rn(A, o, mul_rn(mm, w)) : fma_rn(mm, w, o);
       if constexpr (WX) {
         const T tn = FY || FZ ? fma_rn(A, tt, w) : add_rn(tt, w);
         const T rt = fma_rn(mm, fma_rn(x.op, tn, -mul_rn(x.ir, tt)), o);
@@ -236,7 +250,7 @@ __device__ __forceinline__ void update_row(const bool (&fx)[VN], const AxisCoef<
         O.c[1].v[v] = fma_rn(mm, fma_rn(ry.op, tn, -mul_rn(ry.om, tt)), o);
         t.c[1].v[v] = tn;
       } else {
-        O.c[1].v[v] = fma_rn(mm, w, damp ? mul_rn(A, o) : o);
+        O.c[1].v[v] = FZ ? fma_rn(A, o, mul_rn(mm, w)) : row_o<WX>(f, A, o, mm, w);
       }
     }
     {  // component z: own axis z, next x, previous y
@@ -258,7 +272,7 @@ __device__ __forceinline__ void update_row(const bool (&fx)[VN], const AxisCoef<
         O.c[2].v[v] = fma_rn(mm, fma_rn(zop, tn, -mul_rn(zom, tt)), o);
         t.c[2].v[v] = tn;
       } else {
-        O.c[2].v[v] = fma_rn(mm, w, damp ? mul_rn(A, o) : o);
+        O.c[2].v[v] = FY ? fma_rn(A, o, mul_rn(mm, w)) : row_o<WX>(f, A, o, mm, w);
       }
     }
   }
