@@ -292,13 +292,9 @@ __global__ void __launch_bounds__(kLeanThreads, (VIEW == 2 ? kLeanMinBlocks<T> -
       nb1 = c1;
       const AxisCoef<T> zt = ztab[k - k0];  // read where fz
       bool sp[VN] = {}, anysp = false;
-      Cells<T, VN> w;  // read with the class words, not after them
       if (tf) {
         constexpr uint32_t kSp = H ? kSpecialH : kSpecialE;
         if (sizeof(T) == 4) read_cls();
-        if (anyfx) w.c[0] = get(p.W[0], 2128);
-        if (fy) w.c[1] = get(p.W[1], 2129);
-        if (fz) w.c[2] = get(p.W[2], 2119);
 #pragma unroll
         for (int v = 0; v < VN; ++v) {
           sp[v] = x0 + v < p.nx && ((v ? cls.y : cls.x) & kSp) != 0;
@@ -329,6 +325,10 @@ __global__ void __launch_bounds__(kLeanThreads, (VIEW == 2 ? kLeanMinBlocks<T> -
             t.c[c].v[v] = sp[v] ? tn : t.c[c].v[v];
           }
       } else if (anysp) {
+        Cells<T, VN> w;
+        if (anyfx) w.c[0] = get(p.W[0], 2128);
+        if (fy) w.c[1] = get(p.W[1], 2129);
+        if (fz) w.c[2] = get(p.W[2], 2119);
         RedAxis<T> rz{false, T(1), T(1), T(1), T(1)};
         if (fz) rz = {true, zt.s, zt.om, zt.ir, zt.op};
         update_special_cells<T, VN>(sp, fxv, p.ax[0] + x0, p.ax[1] + j, fz ? p.ax[2][k].s : T(0), xtab + col, ry, rz, K,
