@@ -314,17 +314,7 @@ __global__ void __launch_bounds__(kLeanThreads, (VIEW == 2 ? kLeanMinBlocks<T> -
               if (derived(c, v)) O.c[c].v[v] = t.c[c].v[v];
         }
       }
-      if (anysp && !(anyfx || fy || fz)) {
-        // the most common special cells, a source outside the CPML: T += K, O = m·T
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-          for (int v = 0; v < VN; ++v) {
-            const T tn = add_rn(t.c[c].v[v], K.c[c].v[v]);
-            O.c[c].v[v] = sp[v] ? mul_rn(m.c[c].v[v], tn) : fma_rn(m.c[c].v[v], K.c[c].v[v], O.c[c].v[v]);
-            t.c[c].v[v] = sp[v] ? tn : t.c[c].v[v];
-          }
-      } else if (anysp) {
+      if (anysp) {
         Cells<T, VN> w;
         if (anyfx) w.c[0] = get(p.W[0], 2128);
         if (fy) w.c[1] = get(p.W[1], 2129);
