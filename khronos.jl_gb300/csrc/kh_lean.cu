@@ -490,8 +490,6 @@ void launch_expand_state(bool h_half, const HalfStepParams<T>& p, bool o_kept, v
   else expand_state_kernel<T, false><<<cell_grid(p), 128, 0, st>>>(p, o_kept);
 }
 
-// O of the CPML cells where it is the state into the array of T, free there (KeepArgs):
-// one thread per cell of the absorber's layers.
 // Cell u of the layers: its indices and its place in the padded arrays.
 template <typename T>
 __device__ __forceinline__ long long layer_cell(const KeepArgs<T>& a, long long u, int (&at)[3]) {
@@ -512,6 +510,8 @@ __device__ __forceinline__ long long layer_cell(const KeepArgs<T>& a, long long 
   return a.origin + at[2] * a.plane + at[1] * a.pitch + at[0];
 }
 
+// O of the CPML cells where it is the state into the array of T, free there (KeepArgs):
+// one thread per cell of the absorber's layers.
 template <typename T>
 __global__ void __launch_bounds__(256) keep_state_kernel(const __grid_constant__ KeepArgs<T> a, bool from_t) {
   const KeepHalf<T>& h = a.half[blockIdx.y];
